@@ -102,6 +102,7 @@ msf_status msf_context_destroy(msf_context* ctx) {
   cudaStreamSynchronize(ctx->stream);
   ctx->tw64.clear();
   ctx->tw32.clear();
+  ctx->tw_pair.clear();
   {  // buffers released after this point free their memory directly
     std::lock_guard<std::mutex> lock(ctx->pool->m);
     ctx->pool->closed = true;

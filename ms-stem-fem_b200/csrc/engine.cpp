@@ -168,7 +168,33 @@ msf_status msf_context::twiddles(int n, bool want64, const void** out) {
   return MSF_OK;
 }
 
+msf_status msf_context::col_twiddles(int n, const void** out) {
+  if (fp64) return twiddles(n, true, out);
+  auto it = tw_pair.find(n);
+  if (it == tw_pair.end()) {
+    std::vector<float> f;
+    fill_pair_twiddles(n, f);
+    DevBuf b;
+    MSF_TRY(upload(this, &b, f));
+    it = tw_pair.emplace(n, std::move(b)).first;
+  }
+  *out = it->second.p;
+  return MSF_OK;
+}
+
 namespace msf {
+
+cudaError_t encode_col_map(bool fp64, void* psi, int nb, const Grid& g, void* map) {
+  return fp64 ? encode_column_map(psi, nb, g.nx, g.ny, map)
+              : encode_pair_map(psi, nb, g.nx, g.ny, map);
+}
+
+cudaError_t launch_col_slice(bool fp64, bool pipe_col, bool last, const PassArgs& a,
+                             const void* map, int* err, cudaStream_t s) {
+  if (!fp64) return launch_col_pair(a, last, map, err, s);
+  return pipe_col ? launch_col_slice_pipe(a, last, map, err, s)
+                  : launch_col(last ? COL_SLICE_LAST : COL_SLICE, a, s);
+}
 
 namespace {
 
@@ -188,9 +214,9 @@ msf_status fft2d_f64(msf_context* ctx, const Grid& g, double* planes, int nb, bo
   MSF_TRY(ctx->twiddles(g.nx, true, &a.tw));
   a.scale = scale;
   if (inverse) {
-    MSF_CUDA(launch_col(true, COL_INV, a, ctx->stream));
+    MSF_CUDA(launch_col(COL_INV, a, ctx->stream));
   } else {
-    MSF_CUDA(launch_col(true, COL_FWD, a, ctx->stream));
+    MSF_CUDA(launch_col(COL_FWD, a, ctx->stream));
     if (scale != 1.0)
       MSF_CUDA(launch_scale(planes, a.batch_stride * nb, scale, nullptr, ctx->stream));
   }
@@ -369,7 +395,7 @@ msf_status build_specimen(msf_context* ctx, const msf_grid* gin, const msf_atoms
     for (int j = 0; j < g.ny; ++j) dead[j] = lo[j] == 0 && hi[j] == g.nx;
     spec->n_live_columns = (int)std::count(dead.begin(), dead.end(), 0);
     const bool fp = ctx->fp64;
-    const int T = row_line_threads(g.ny, fp), cols = pipe_cols_for(g.nx, fp);
+    const int T = row_line_threads(g.ny, fp), cols = fp ? pipe_cols_for(g.nx) : col_pair_tile(g.nx);
     if (T > 0 && g.ny / T <= 32 && cols > 0 && spec->n_live_columns < g.ny) {
       std::vector<uint32_t> bits(T, 0u);
       for (int t = 0; t < T; ++t)
@@ -458,7 +484,7 @@ msf_status build_specimen(msf_context* ctx, const msf_grid* gin, const msf_atoms
     MSF_TRY(ctx->twiddles(g.ny, true, &a.tw));
     MSF_CUDA(launch_row(true, ROW_FWD, a, ctx->stream));
     MSF_TRY(ctx->twiddles(g.nx, true, &a.tw));
-    MSF_CUDA(launch_col(true, COL_FWD_MASK_INV, a, ctx->stream));
+    MSF_CUDA(launch_col(COL_FWD_MASK_INV, a, ctx->stream));
     MSF_TRY(ctx->twiddles(g.ny, true, &a.tw));
     a.scale = 1.0 / g.nxny;
     MSF_CUDA(launch_row(true, ROW_INV, a, ctx->stream));
@@ -556,7 +582,7 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
   MSF_TRY(ctx->twiddles(g.ny, fp64, &row.tw));
-  MSF_TRY(ctx->twiddles(g.nx, fp64, &col.tw));
+  MSF_TRY(ctx->col_twiddles(g.nx, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.trans = spec->t.p;
   row.psi0 = psi0.p;
@@ -571,12 +597,13 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
   const int row_sched = !fp64 && staged_row_supported(g.nx, g.ny) && (pipe & MSF_ROW_ALT) ? 1 : 0;
   const bool pipe_row = !fp64 && !staged_row && !row_sched && pipe_supported(g.nx, g.ny) &&
                         (pipe & MSF_PIPE_ROW);
-  const bool pipe_col = pipe_supported(g.nx, g.ny, fp64) && (pipe & MSF_PIPE_COL);
+  const bool pipe_col =
+      !fp64 || (pipe_supported(g.nx, g.ny, true) && (pipe & MSF_PIPE_COL));
   alignas(64) unsigned char col_map[128];
   DevBuf d_err;
   MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), ctx->stream));
-  if (pipe_col) MSF_CUDA(encode_column_map(psi.p, nb, g.nx, g.ny, col_map, fp64));
+  if (pipe_col) MSF_CUDA(encode_col_map(fp64, psi.p, nb, g, col_map));
   if (pipe_col && !pipe_row && spec->n_live_groups > 0) {  // skip removed columns
     row.row_dead_bits = spec->dead_bits.as<uint32_t>();
     row.row_dead_io = 3;  // a slice between the first and the last
@@ -598,8 +625,7 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
                             : launch_row(fp64, rop, row, ctx->stream);
   };
   auto col_pass = [&]() {
-    return pipe_col ? launch_col_slice_pipe(col, false, col_map, d_err.as<int>(), ctx->stream, fp64)
-                    : launch_col(fp64, COL_SLICE, col, ctx->stream);
+    return launch_col_slice(fp64, pipe_col, false, col, col_map, d_err.as<int>(), ctx->stream);
   };
   std::vector<cudaEvent_t> ev(2 * reps + 2);
   for (auto& e : ev) MSF_CUDA(cudaEventCreate(&e));
@@ -729,7 +755,7 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
       v.tw = tw_x;
       v.px = prop64.as<double>() + 2 * (size_t)(g.nx + g.ny) * s;
       v.py = prop64.as<double>() + 2 * (size_t)(g.nx + g.ny) * s + 2 * g.nx;
-      MSF_CUDA(launch_col(true, s + 1 == S ? COL_SLICE_LAST : COL_SLICE, v, ctx->stream));
+      MSF_CUDA(launch_col(s + 1 == S ? COL_SLICE_LAST : COL_SLICE, v, ctx->stream));
       P->setup_launches += 3;
       if (s + 1 < S) {
         v.tw = tw_y;
@@ -814,13 +840,13 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
     MSF_TRY(ctx->twiddles(g.ny, true, &a.tw));
     MSF_CUDA(launch_row(true, ROW_INV, a, ctx->stream));
     MSF_TRY(ctx->twiddles(g.nx, true, &a.tw));
-    MSF_CUDA(launch_col(true, COL_INV, a, ctx->stream));
+    MSF_CUDA(launch_col(COL_INV, a, ctx->stream));
     MSF_CUDA(launch_bw_limit(P->mtf2d.as<double>(), spec->mask_lo.as<int32_t>(),
                              spec->mask_hi.as<int32_t>(), g.nx, g.ny, ctx->stream));
     MSF_TRY(ctx->twiddles(g.ny, true, &a.tw));
     MSF_CUDA(launch_row(true, ROW_FWD, a, ctx->stream));
     MSF_TRY(ctx->twiddles(g.nx, true, &a.tw));
-    MSF_CUDA(launch_col(true, COL_FWD, a, ctx->stream));
+    MSF_CUDA(launch_col(COL_FWD, a, ctx->stream));
     MSF_CUDA(launch_scale(P->mtf2d.as<double>(), plane, 1.0 / g.nxny, nullptr, ctx->stream));
     P->setup_launches += 6;
   }
@@ -856,12 +882,12 @@ msf_status mtf_stage(msf_context* ctx, const RasterPlan& P, bool fp64, const voi
   a.tw = tw_y;
   MSF_CUDA(launch_row(true, ROW_INV, a, st));
   a.tw = tw_x;
-  MSF_CUDA(launch_col(true, COL_INV, a, st));
+  MSF_CUDA(launch_col(COL_INV, a, st));
   MSF_CUDA(launch_mtf_multiply(out, P.mtf2d.as<double>(), plane, nb, 1.0 / g.s, st));
   a.tw = tw_y;
   MSF_CUDA(launch_row(true, ROW_FWD, a, st));
   a.tw = tw_x;
-  MSF_CUDA(launch_col(true, COL_FWD, a, st));
+  MSF_CUDA(launch_col(COL_FWD, a, st));
   MSF_CUDA(launch_scale(out, plane * nb, 1.0 / g.s, nullptr, st));
   MSF_CUDA(launch_bw_limit(out, spec->mask_lo.as<int32_t>(), spec->mask_hi.as<int32_t>(), g.nx,
                            g.ny, st, nb));
@@ -1129,12 +1155,13 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   const int row_sched = !fp64 && staged_row_supported(g.nx, g.ny) && (pipe & MSF_ROW_ALT) ? 1 : 0;
   const bool pipe_row = !fp64 && !staged_row && !row_sched && pipe_supported(g.nx, g.ny) &&
                         (pipe & MSF_PIPE_ROW);
-  const bool pipe_col = pipe_supported(g.nx, g.ny, fp64) && (pipe & MSF_PIPE_COL);
+  const bool pipe_col =
+      !fp64 || (pipe_supported(g.nx, g.ny, true) && (pipe & MSF_PIPE_COL));
   alignas(64) unsigned char col_map[128];
   DevBuf d_err;
   MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), ctx->stream));
-  if (pipe_col) MSF_CUDA(encode_column_map(psi.p, B, g.nx, g.ny, col_map, fp64));
+  if (pipe_col) MSF_CUDA(encode_col_map(fp64, psi.p, B, g, col_map));
 
   PassArgs row, col;
   if (pipe_col && !pipe_row && spec->n_live_groups > 0) {  // skip removed columns
@@ -1147,7 +1174,7 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
   MSF_TRY(ctx->twiddles(g.ny, fp64, &row.tw));
-  MSF_TRY(ctx->twiddles(g.nx, fp64, &col.tw));
+  MSF_TRY(ctx->col_twiddles(g.nx, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.prefetch_tables = (!fp64 && (pipe & MSF_ROW_PREFETCH)) ? 1 : 0;
   if (!fp64 && !staged_row && row_sched == 0 && !pipe_row && (pipe & MSF_ROW_L2AHEAD))
@@ -1206,11 +1233,8 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
       if (timing_passes) MSF_CUDA(cudaEventRecord(pass_ev[3 * s + 1], ctx->stream));
       col.px = pbase + prop_stride * s;
       col.py = pbase + prop_stride * s + cbytes * g.nx;
-      if (pipe_col)
-        MSF_CUDA(launch_col_slice_pipe(col, s + 1 == S, col_map, d_err.as<int>(), ctx->stream,
-                                       fp64));
-      else
-        MSF_CUDA(launch_col(fp64, s + 1 == S ? COL_SLICE_LAST : COL_SLICE, col, ctx->stream));
+      MSF_CUDA(launch_col_slice(fp64, pipe_col, s + 1 == S, col, col_map, d_err.as<int>(),
+                                ctx->stream));
       if (timing_passes) MSF_CUDA(cudaEventRecord(pass_ev[3 * s + 2], ctx->stream));
     }
     SplitK sk;
@@ -1433,7 +1457,7 @@ msf_status run_raster_plain(msf_context* ctx, const msf_specimen* spec,
     a.tw = tw_y;
     MSF_CUDA(launch_row(true, inverse ? ROW_INV : ROW_FWD, a, st));
     a.tw = tw_x;
-    MSF_CUDA(launch_col(true, inverse ? COL_INV : COL_FWD, a, st));
+    MSF_CUDA(launch_col(inverse ? COL_INV : COL_FWD, a, st));
     return MSF_OK;
   };
   const double* t0 = spec->t.as<double>();

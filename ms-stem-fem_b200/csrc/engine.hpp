@@ -105,7 +105,8 @@ struct msf_context {
   int64_t allocated() const { return pool->live; }
   int64_t h2d_bytes = 0, d2h_bytes = 0;
   cudaStream_t stream = nullptr;
-  std::map<int, msf::DevBuf> tw64, tw32;  // twiddle tables per length
+  // twiddle tables per length; tw_pair: the FP32 column pass's (fft_pair.cuh)
+  std::map<int, msf::DevBuf> tw64, tw32, tw_pair;
   // autotuned launch tiling per grid (nx, ny): probes per launch and the
   // pipelined-pass mask (msf_tune, or imported wisdom)
   struct Tuned {
@@ -149,6 +150,8 @@ struct msf_context {
   bool keep_potentials = false;
   msf_status alloc(msf::DevBuf* b, size_t bytes);
   msf_status twiddles(int n, bool fp64, const void** out);
+  // the table of the context's column slice pass
+  msf_status col_twiddles(int n, const void** out);
 };
 
 struct msf_specimen {
@@ -251,6 +254,7 @@ msf_status run_partial(msf_context* ctx, const msf_specimen* spec, const msf_opt
                        int64_t p_end, double* amp, double* inten, double* acc_a,
                        double* acc_i, msf_results* info);
 
+struct PassArgs;
 msf_status build_specimen(msf_context* ctx, const msf_grid* grid, const msf_atoms* atoms,
                           msf_specimen* spec);
 msf_status run_raster(msf_context* ctx, const msf_specimen* spec, const msf_optics* optics,
@@ -262,8 +266,12 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
 msf_status run_batch(msf_context* ctx, int n, const msf_specimen* const* specs,
                      const msf_optics* optics, const msf_raster* rasters,
                      const msf_detect* detects, msf_results* results, int slots);
+// The tensor map and launch of the context's batched column slice pass: FP32
+// contexts always, FP64 ones when `pipe_col` (else the plain kernel, no map).
+cudaError_t encode_col_map(bool fp64, void* psi, int nb, const Grid& g, void* map);
+cudaError_t launch_col_slice(bool fp64, bool pipe_col, bool last, const PassArgs& a,
+                             const void* map, int* err, cudaStream_t s);
 int lane_slots(int want, int64_t plane, int lanes, int64_t probes);
-struct PassArgs;
 // The plain FP32 split-wave row pass's L2 prefetch ahead (MSF_ROW_L2AHEAD)
 // for rows of `spec`'s grid: distance and live element ranges.
 void set_row_ahead(const msf_context* ctx, const msf_specimen* spec, PassArgs* row);

@@ -89,7 +89,8 @@ constexpr int row_lines() {
 }
 
 // Columns per CTA of a column pass: as many as fit MSF_COL_THREADS threads
-// (16 FP32 / 8 FP64 columns give 128-byte row segments).
+// (8 FP64 columns give 128-byte row segments; the FP32 column pass is
+// kernels_col32.cu).
 template <typename Real, int N>
 constexpr int col_cols() {
   using Sh = Shape<N, Real>;
@@ -358,21 +359,6 @@ col_kernel(const PassArgs a) {
   C* sm = smem + c * SM::stride;
   const C* tw = static_cast<const C*>(a.tw);
   auto sync = [] { __syncthreads(); };
-  // slot batch: this CTA's probe brings its own mask, propagator and step
-  const int32_t* mask_lo = a.mask_lo;
-  const int32_t* mask_hi = a.mask_hi;
-  const void* px_v = a.px;
-  const void* py_v = a.py;
-  [[maybe_unused]] bool stop_in_k = OP == COL_SLICE_LAST;
-  if constexpr (OP == COL_SLOTS) {
-    const SlotPass& sp = a.slots[b];
-    if (sp.op == SLOT_IDLE) return;
-    mask_lo = sp.mask_lo;
-    mask_hi = sp.mask_hi;
-    px_v = sp.px;
-    py_v = sp.py;
-    stop_in_k = sp.last != 0;
-  }
   C v[E];
 #pragma unroll
   for (int m = 0; m < E; ++m) v[m] = col[(int64_t)(t + T * m) * ny];
@@ -384,7 +370,7 @@ col_kernel(const PassArgs a) {
   } else {
     fft_line<Sh, false>(v, sm, t, tw, sync);
     if constexpr (OP != COL_FWD) {
-      const int lo = __ldg(mask_lo + j), hi = __ldg(mask_hi + j);
+      const int lo = __ldg(a.mask_lo + j), hi = __ldg(a.mask_hi + j);
       if constexpr (OP == COL_FWD_MASK_INV) {
 #pragma unroll
         for (int m = 0; m < E; ++m) {
@@ -393,8 +379,8 @@ col_kernel(const PassArgs a) {
         }
       } else {
         const Real is = (Real)a.inv_s;
-        const C pyj = __ldg(static_cast<const C*>(py_v) + j);
-        const C* px = static_cast<const C*>(px_v);
+        const C pyj = __ldg(static_cast<const C*>(a.py) + j);
+        const C* px = static_cast<const C*>(a.px);
 #pragma unroll
         for (int m = 0; m < E; ++m) {
           if (m % kLoadChunk == 0) load_fence();
@@ -409,8 +395,6 @@ col_kernel(const PassArgs a) {
       }
       if constexpr (OP == COL_FWD_MASK_INV || OP == COL_SLICE)
         fft_line<Sh, true>(v, sm, t, tw, sync);
-      if constexpr (OP == COL_SLOTS)
-        if (!stop_in_k) fft_line<Sh, true>(v, sm, t, tw, sync);
     }
   }
 #pragma unroll
@@ -1097,22 +1081,13 @@ cudaError_t launch_row_split_alt(const PassArgs& a, cudaStream_t s) {
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_col(bool fp64, ColOp op, const PassArgs& a, cudaStream_t s) {
-  if (fp64) {
-    switch (op) {
-      case COL_FWD: return col_dispatch<double, COL_FWD>(a, s);
-      case COL_INV: return col_dispatch<double, COL_INV>(a, s);
-      case COL_FWD_MASK_INV: return col_dispatch<double, COL_FWD_MASK_INV>(a, s);
-      case COL_SLICE: return col_dispatch<double, COL_SLICE>(a, s);
-      case COL_SLICE_LAST: return col_dispatch<double, COL_SLICE_LAST>(a, s);
-    }
-  } else {
-    switch (op) {
-      case COL_SLICE: return col_dispatch<float, COL_SLICE>(a, s);
-      case COL_SLICE_LAST: return col_dispatch<float, COL_SLICE_LAST>(a, s);
-      case COL_SLOTS: return col_dispatch<float, COL_SLOTS>(a, s);
-      default: return cudaErrorInvalidValue;
-    }
+cudaError_t launch_col(ColOp op, const PassArgs& a, cudaStream_t s) {
+  switch (op) {
+    case COL_FWD: return col_dispatch<double, COL_FWD>(a, s);
+    case COL_INV: return col_dispatch<double, COL_INV>(a, s);
+    case COL_FWD_MASK_INV: return col_dispatch<double, COL_FWD_MASK_INV>(a, s);
+    case COL_SLICE: return col_dispatch<double, COL_SLICE>(a, s);
+    case COL_SLICE_LAST: return col_dispatch<double, COL_SLICE_LAST>(a, s);
   }
   return cudaErrorInvalidValue;
 }

@@ -65,7 +65,6 @@ enum ColOp : int {
   COL_FWD_MASK_INV = 2,  // forward DFT, band-limit mask, inverse DFT
   COL_SLICE = 3,         // fwd DFT, /s, mask, propagator, inverse DFT
   COL_SLICE_LAST = 4,    // fwd DFT, /s, mask, propagator (stay in k-space)
-  COL_SLOTS = 5,         // COL_SLICE or COL_SLICE_LAST per slot (FP32)
 };
 
 // One probe slot's step in a slot batch: probes of different specimens (of
@@ -108,7 +107,7 @@ struct PassArgs {
   // split-wave row passes: vacuum wave entering this slice, [nx][ny]
   // complex, in the same scale as the inverse-transformed buffer
   const void* psi0 = nullptr;
-  // slot batches (ROW_SLOTS, COL_SLOTS, pipelined column pass): [nb]
+  // slot batches (ROW_SLOTS, the FP32 column pass): [nb]
   const SlotPass* slots = nullptr;
   // Columns the band limit removes entirely (lo = 0, hi = nx: no kx kept):
   // the slice row passes store zeros there (bit m of word t: column
@@ -158,8 +157,8 @@ struct SplitK {
 bool supported_length(int n);
 // Threads per line of the row transform of length n (its T); 0 if unsupported.
 int row_line_threads(int n, bool fp64);
-// Columns per tile of the pipelined column pass (0 if unsupported).
-int pipe_cols_for(int nx, bool fp64);
+// Columns per tile of the pipelined FP64 column pass (0 if unsupported).
+int pipe_cols_for(int nx);
 cudaError_t launch_row(bool fp64, RowOp op, const PassArgs& a, cudaStream_t s);
 // CTAs of the FP32 split-wave row pass (ROW_SPLIT, default schedule) that
 // the current device holds at once for rows of length ny (0 if
@@ -170,11 +169,11 @@ int row_split_resident_ctas(int ny);
 // in that schedule's layout, staged_row_threads(ny, 1)); row lengths
 // 256..2048.
 cudaError_t launch_row_split_alt(const PassArgs& a, cudaStream_t s);
-cudaError_t launch_col(bool fp64, ColOp op, const PassArgs& a, cudaStream_t s);
+cudaError_t launch_col(ColOp op, const PassArgs& a, cudaStream_t s);  // FP64
 
 // ---- persistent TMA-pipelined slice passes (kernels_pipe.cu) ----
-// The column pass: FP32 grids with sides 256..2048, FP64 grids with sides
-// 256..1024; the split-wave row pass: FP32 only.
+// The FP64 column pass: grids with sides 256..1024; the split-wave row pass
+// (FP32 only): 256..2048.
 bool pipe_supported(int nx, int ny, bool fp64 = false);
 // Split-wave row pass for slices after the first; *err set to 1 if a copy
 // never arrived (bounded wait).
@@ -194,14 +193,24 @@ bool staged_row_supported(int nx, int ny);
 int staged_row_threads(int ny, int schedule);
 cudaError_t launch_row_split_staged(const PassArgs& a, int* err, cudaStream_t s,
                                     int schedule = 0);
-// Column slice pass (COL_SLICE, or COL_SLICE_LAST when `last`; per slot
-// when a.slots is set); `tensor_map` from encode_column_map over the same
-// batch buffer.
+// FP64 column slice pass (COL_SLICE, or COL_SLICE_LAST when `last`);
+// `tensor_map` from encode_column_map over the same batch buffer.
 cudaError_t launch_col_slice_pipe(const PassArgs& a, bool last, const void* tensor_map,
-                                  int* err, cudaStream_t s, bool fp64 = false);
-// Encode the 2-D tensor map (128 bytes) the column pass loads tiles with.
-cudaError_t encode_column_map(void* psi, int nb, int nx, int ny, void* map_out,
-                              bool fp64 = false);
+                                  int* err, cudaStream_t s);
+// Encode the 2-D tensor map (128 bytes) the FP64 column pass loads tiles with.
+cudaError_t encode_column_map(void* psi, int nb, int nx, int ny, void* map_out);
+
+// ---- the FP32 column pass (kernels_col32.cu), sides 64..4096 ----
+// COL_SLICE, or COL_SLICE_LAST when `last`, or per slot when a.slots is set;
+// a.tw from fill_pair_twiddles, `tensor_map` (128 bytes) from encode_pair_map
+// over the same batch buffer; *err set to 1 if a copy never arrived (bounded
+// wait).  The columns of a live group: col_pair_tile(nx) neighbours.
+cudaError_t launch_col_pair(const PassArgs& a, bool last, const void* tensor_map, int* err,
+                            cudaStream_t s);
+int col_pair_tile(int nx);  // 0 if unsupported
+cudaError_t encode_pair_map(void* psi, int nb, int nx, int ny, void* map_out);
+// Twiddles of the packed transform of length n, stage by stage (fft_pair.cuh).
+void fill_pair_twiddles(int n, std::vector<float>& out);
 
 // Twiddle table e^{-2 pi i m / n}, m < n, computed in FP64 on the host.
 void fill_twiddles(int n, double* host_interleaved /* 2n */);

@@ -1,4 +1,5 @@
-// Persistent, TMA-pipelined versions of the two FP32 slice passes.
+// Persistent, TMA-pipelined slice passes: the FP64 column pass and variants
+// of the FP32 split-wave row pass.
 //
 // One CTA per SM walks a list of work items (a group of rows, or a group of
 // columns, of one probe).  While it transforms item k out of one shared
@@ -15,6 +16,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include "async_copy.cuh"
 #include "fft_core.cuh"
 #include "kernels.h"
 
@@ -22,54 +24,6 @@ namespace msf {
 
 namespace {
 
-constexpr uint32_t kSpinLimit = 1u << 22;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-  for (uint32_t it = 0; it < kSpinLimit; ++it)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes,
-                                         uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void tile_g2s(void* dst, const CUtensorMap* map, int x, int y,
-                                         uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
 // A wavefield element loaded once per pass: not allocated in L1, which
 // then keeps the twiddle table (read by every stage of every line).
 __device__ __forceinline__ float2 ld_once(const float2* p) {
@@ -77,21 +31,6 @@ __device__ __forceinline__ float2 ld_once(const float2* p) {
   asm("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
   return v;
 }
-__device__ __forceinline__ void fence_proxy_async() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Thread 0 waits (bounded) for the buffer's phase, the CTA learns the
-// outcome through shared memory, then every thread observes the completed
-// phase itself (acquiring the copied data).
-__device__ __forceinline__ bool cta_wait(uint64_t* bar, uint32_t parity, int* flag_smem) {
-  if (threadIdx.x == 0) *flag_smem = mbar_wait_bounded(bar, parity) ? 1 : 0;
-  __syncthreads();
-  const bool ok = *flag_smem != 0;
-  if (ok) mbar_wait_bounded(bar, parity);
-  return ok;
-}
-
 // ------------------------------------------------------- row pass (split) --
 template <int N, int LINES>
 __global__ void __launch_bounds__(LINES * Shape<N, float>::T, 1)
@@ -318,11 +257,9 @@ constexpr int col_pipe_min_ctas(int threads) {
   return threads >= MSF_COL_PIPE_THREADS_PER_SM ? 1 : MSF_COL_PIPE_THREADS_PER_SM / threads;
 }
 
-// Real: float (the split-wave passes) or double (FP64 runs; a complex value
-// is then two 8-byte tensor-map elements).  SLOTS (FP32 only): every probe
-// of the batch brings its own mask, propagator and step (PassArgs::slots);
-// LAST is then taken per probe from its slot.
-template <typename Real, int N, int COLS, bool LAST, bool SLOTS>
+// FP64 runs (a complex value is two 8-byte tensor-map elements); the FP32
+// column pass is kernels_col32.cu.
+template <typename Real, int N, int COLS, bool LAST>
 __global__ void __launch_bounds__(COLS * Shape<N, Real>::T,
                                   col_pipe_min_ctas(COLS * Shape<N, Real>::T))
 col_slice_pipe_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap, int* err) {
@@ -372,10 +309,6 @@ col_slice_pipe_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap
   int k = 0;
   for (; item < items; ++k, item += gridDim.x) {
     const int w = k & 1;
-    // a slot batch reads its slot entry before the tile wait, so that the
-    // load overlaps the copy instead of following it
-    SlotPass sp{};
-    if constexpr (SLOTS) sp = a.slots[item % a.nb];
     if (!cta_wait(&bars[w], parity[w], &flag)) {
       if (threadIdx.x == 0) {
         atomicExch(err, 1);
@@ -387,20 +320,7 @@ col_slice_pipe_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap
     const int gi = item / a.nb, b = item - gi * a.nb;
     const int g = group_of(gi);
     const int j = g * COLS + c;
-    const int32_t* mask_lo = a.mask_lo;
-    const int32_t* mask_hi = a.mask_hi;
-    const C* pxb = px;
-    const C* pyb = static_cast<const C*>(a.py);
-    bool idle = false, stop_in_k = LAST;
-    if constexpr (SLOTS) {
-      idle = sp.op == SLOT_IDLE;
-      mask_lo = sp.mask_lo;
-      mask_hi = sp.mask_hi;
-      pxb = static_cast<const C*>(sp.px);
-      pyb = static_cast<const C*>(sp.py);
-      stop_in_k = sp.last != 0;
-    }
-    if (!idle) {
+    {
       C* base = bufs + w * BUF;
       C v[E];
 #pragma unroll
@@ -410,20 +330,20 @@ col_slice_pipe_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap
       if constexpr (Sh::S == 1) __syncthreads();
       C* sm = base + c * SM::stride;
       fft_line<Sh, false>(v, sm, t, tw, sync);
-      const int lo = __ldg(mask_lo + j), hi = __ldg(mask_hi + j);
-      const C pyj = __ldg(pyb + j);
+      const int lo = __ldg(a.mask_lo + j), hi = __ldg(a.mask_hi + j);
+      const C pyj = __ldg(static_cast<const C*>(a.py) + j);
 #pragma unroll
       for (int m = 0; m < E; ++m) {
         if (m % kLoadChunk == 0) load_fence();
         const int i = t + T * m;
         if (i < lo || i >= hi) {
-          const C p = cmul(__ldg(pxb + i), pyj);
+          const C p = cmul(__ldg(px + i), pyj);
           v[m] = cmul(p, cscale(v[m], is));
         } else {
           v[m] = C{Real(0), Real(0)};
         }
       }
-      if (!stop_in_k) fft_line<Sh, true>(v, sm, t, tw, sync);
+      if constexpr (!LAST) fft_line<Sh, true>(v, sm, t, tw, sync);
       C* col = static_cast<C*>(a.psi) + (int64_t)b * a.batch_stride + j;
 #pragma unroll
       for (int m = 0; m < E; ++m) col[(int64_t)(t + T * m) * a.ny] = v[m];
@@ -490,7 +410,7 @@ cudaError_t row_staged_launch(const PassArgs& a, int* err, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <typename Real, int N, bool LAST, bool SLOTS = false>
+template <typename Real, int N, bool LAST>
 cudaError_t col_pipe_launch(const PassArgs& a, const CUtensorMap& map, int* err,
                             cudaStream_t s) {
   constexpr int CC = pipe_cols<Real, N>();
@@ -501,7 +421,7 @@ cudaError_t col_pipe_launch(const PassArgs& a, const CUtensorMap& map, int* err,
   // resident CTAs per SM, found once per device after raising the limit
   static PerDevice configured;
   static std::atomic<int> per_sm_dev[64];
-  auto k = col_slice_pipe_kernel<Real, N, CC, LAST, SLOTS>;
+  auto k = col_slice_pipe_kernel<Real, N, CC, LAST>;
   const int dev = current_device();
   int per_sm = (dev >= 0 && dev < 64) ? per_sm_dev[dev].load() : 0;
   if (configured.needed(dev) || per_sm < 1) {
@@ -530,20 +450,11 @@ bool pipe_supported(int nx, int ny, bool fp64) {
   return ok(nx) && ok(ny);
 }
 
-int pipe_cols_for(int nx, bool fp64) {
-  if (fp64) {
-    switch (nx) {
-      case 256: return pipe_cols<double, 256>();
-      case 512: return pipe_cols<double, 512>();
-      case 1024: return pipe_cols<double, 1024>();
-    }
-    return 0;
-  }
+int pipe_cols_for(int nx) {
   switch (nx) {
-    case 256: return pipe_cols<float, 256>();
-    case 512: return pipe_cols<float, 512>();
-    case 1024: return pipe_cols<float, 1024>();
-    case 2048: return pipe_cols<float, 2048>();
+    case 256: return pipe_cols<double, 256>();
+    case 512: return pipe_cols<double, 512>();
+    case 1024: return pipe_cols<double, 1024>();
   }
   return 0;
 }
@@ -593,39 +504,20 @@ cudaError_t launch_row_split_staged(const PassArgs& a, int* err, cudaStream_t s,
 }
 
 cudaError_t launch_col_slice_pipe(const PassArgs& a, bool last, const void* tensor_map,
-                                  int* err, cudaStream_t s, bool fp64) {
+                                  int* err, cudaStream_t s) {
   const CUtensorMap& m = *static_cast<const CUtensorMap*>(tensor_map);
-  if (fp64) {
-    if (a.slots) return cudaErrorInvalidValue;
-    switch (a.nx) {
-      case 256: return last ? col_pipe_launch<double, 256, true>(a, m, err, s) : col_pipe_launch<double, 256, false>(a, m, err, s);
-      case 512: return last ? col_pipe_launch<double, 512, true>(a, m, err, s) : col_pipe_launch<double, 512, false>(a, m, err, s);
-      case 1024: return last ? col_pipe_launch<double, 1024, true>(a, m, err, s) : col_pipe_launch<double, 1024, false>(a, m, err, s);
-    }
-    return cudaErrorInvalidValue;
-  }
-  if (a.slots) {
-    switch (a.nx) {
-      case 256: return col_pipe_launch<float, 256, false, true>(a, m, err, s);
-      case 512: return col_pipe_launch<float, 512, false, true>(a, m, err, s);
-      case 1024: return col_pipe_launch<float, 1024, false, true>(a, m, err, s);
-      case 2048: return col_pipe_launch<float, 2048, false, true>(a, m, err, s);
-    }
-    return cudaErrorInvalidValue;
-  }
   switch (a.nx) {
-    case 256: return last ? col_pipe_launch<float, 256, true>(a, m, err, s) : col_pipe_launch<float, 256, false>(a, m, err, s);
-    case 512: return last ? col_pipe_launch<float, 512, true>(a, m, err, s) : col_pipe_launch<float, 512, false>(a, m, err, s);
-    case 1024: return last ? col_pipe_launch<float, 1024, true>(a, m, err, s) : col_pipe_launch<float, 1024, false>(a, m, err, s);
-    case 2048: return last ? col_pipe_launch<float, 2048, true>(a, m, err, s) : col_pipe_launch<float, 2048, false>(a, m, err, s);
+    case 256: return last ? col_pipe_launch<double, 256, true>(a, m, err, s) : col_pipe_launch<double, 256, false>(a, m, err, s);
+    case 512: return last ? col_pipe_launch<double, 512, true>(a, m, err, s) : col_pipe_launch<double, 512, false>(a, m, err, s);
+    case 1024: return last ? col_pipe_launch<double, 1024, true>(a, m, err, s) : col_pipe_launch<double, 1024, false>(a, m, err, s);
   }
   return cudaErrorInvalidValue;
 }
 
-// Tensor map over a batch of complex planes [nb*nx rows][ny columns] of
-// 8-byte elements (one per FP32 complex value, two per FP64 one), box
-// {cols, min(256, nx)} rows; no multicast, no swizzle.
-cudaError_t encode_column_map(void* psi, int nb, int nx, int ny, void* map_out, bool fp64) {
+// Tensor map over a batch of FP64 complex planes [nb*nx rows][ny columns],
+// two 8-byte elements a value, box {cols, min(256, nx)} rows; no multicast,
+// no swizzle.
+cudaError_t encode_column_map(void* psi, int nb, int nx, int ny, void* map_out) {
   // looked up once per process (a thread-safe static: lanes of the request
   // loop encode maps from their worker thread)
   static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
@@ -637,9 +529,9 @@ cudaError_t encode_column_map(void* psi, int nb, int nx, int ny, void* map_out, 
                : nullptr;
   }();
   if (!encode) return cudaErrorNotSupported;
-  const int cols = pipe_cols_for(nx, fp64);
+  const int cols = pipe_cols_for(nx);
   if (!cols) return cudaErrorInvalidValue;
-  const int epc = fp64 ? 2 : 1;  // 8-byte elements per complex value
+  const int epc = 2;  // 8-byte elements per complex value
   cuuint64_t dims[2] = {(cuuint64_t)ny * epc, (cuuint64_t)nx * (cuuint64_t)nb};
   cuuint64_t strides[1] = {(cuuint64_t)ny * 8 * epc};
   cuuint32_t box[2] = {(cuuint32_t)(cols * epc), (cuuint32_t)(nx < 256 ? nx : 256)};

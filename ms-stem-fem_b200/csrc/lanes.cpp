@@ -71,19 +71,18 @@ msf_status Lane::init() {
   for (auto& e : ring_ev_) MSF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   MSF_TRY(ctx_->alloc(&err_, sizeof(int)));
   MSF_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(int), stream_));
-  pipe_col_ = (ctx_->pipe & MSF_PIPE_COL) && pipe_supported(nx_, ny_);
   // MSF_LANE_GROUPS=0: every step runs the slot passes (the two paths give
   // the same bits; the switch lets tests and benchmarks compare them)
   const char* u = std::getenv("MSF_LANE_GROUPS");
   groups_ok_ = !(u && u[0] == '0');
-  if (pipe_col_) MSF_CUDA(encode_column_map(psi_.p, B_, nx_, ny_, col_map_));
+  MSF_CUDA(encode_pair_map(psi_.p, B_, nx_, ny_, col_map_));
   row_.psi = col_.psi = psi_.p;
   row_.batch_stride = col_.batch_stride = plane_;
   row_.nb = col_.nb = B_;
   row_.nx = col_.nx = nx_;
   row_.ny = col_.ny = ny_;
   MSF_TRY(ctx_->twiddles(ny_, false, &row_.tw));
-  MSF_TRY(ctx_->twiddles(nx_, false, &col_.tw));
+  MSF_TRY(ctx_->col_twiddles(nx_, &col_.tw));
   row_.slots = col_.slots = static_cast<const SlotPass*>(table_.p);
   row_.prefetch_tables = (ctx_->pipe & MSF_ROW_PREFETCH) ? 1 : 0;
   slot_.assign(B_, Slot{});
@@ -116,7 +115,7 @@ msf_status Lane::add(SlotJob* job) {
   const msf_specimen* spec = job->plan.spec;
   if (!skip_decided_) {
     skip_decided_ = true;
-    if (pipe_col_ && spec->n_live_groups > 0) {
+    if (spec->n_live_groups > 0) {
       MSF_TRY(ctx_->alloc(&dead_bits_, spec->dead_bits.bytes));
       MSF_TRY(ctx_->alloc(&live_groups_, spec->live_groups.bytes));
       MSF_CUDA(cudaMemcpyAsync(dead_bits_.p, spec->dead_bits.p, spec->dead_bits.bytes,
@@ -167,10 +166,7 @@ msf_status Lane::add(SlotJob* job) {
 
 msf_status Lane::launch_passes() {
   MSF_CUDA(launch_row(false, ROW_SLOTS, row_, stream_));
-  if (pipe_col_)
-    MSF_CUDA(launch_col_slice_pipe(col_, false, col_map_, err_.as<int>(), stream_));
-  else
-    MSF_CUDA(launch_col(false, COL_SLOTS, col_, stream_));
+  MSF_CUDA(launch_col_pair(col_, false, col_map_, err_.as<int>(), stream_));
   return MSF_OK;
 }
 
@@ -207,19 +203,15 @@ msf_status Lane::launch_group(const SlotJob* job, int s, int base, int nb) {
   col.py = static_cast<const char*>(col.px) + 8 * (size_t)nx_;
   col.mask_lo = spec->mask_lo.as<int32_t>();
   col.mask_hi = spec->mask_hi.as<int32_t>();
-  if (pipe_col_) {
-    // the lane's tensor map starts at wavefield 0; a group further in gets
-    // its own (encoding is a host call that allocates nothing)
-    alignas(64) unsigned char map[128];
-    const void* m = col_map_;
-    if (base != 0) {
-      MSF_CUDA(encode_column_map(col.psi, nb, nx_, ny_, map));
-      m = map;
-    }
-    MSF_CUDA(launch_col_slice_pipe(col, last, m, err_.as<int>(), stream_));
-  } else {
-    MSF_CUDA(launch_col(false, last ? COL_SLICE_LAST : COL_SLICE, col, stream_));
+  // the lane's tensor map starts at wavefield 0; a group further in gets
+  // its own (encoding is a host call that allocates nothing)
+  alignas(64) unsigned char map[128];
+  const void* m = col_map_;
+  if (base != 0) {
+    MSF_CUDA(encode_pair_map(col.psi, nb, nx_, ny_, map));
+    m = map;
   }
+  MSF_CUDA(launch_col_pair(col, last, m, err_.as<int>(), stream_));
   return MSF_OK;
 }
 

@@ -105,7 +105,6 @@ class Lane {
   cudaStream_t stream_ = nullptr;
   DevBuf psi_, table_, partial_, err_;
   int max_chunks_ = 0;
-  bool pipe_col_ = false;
   // removed-column skipping: on while every raster the lane was given has
   // the same removed columns (the first one's); off for good otherwise
   bool skip_ = false, skip_decided_ = false;

@@ -131,10 +131,10 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
   cudaStream_t st = ctx->stream;
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
 
-  const bool pipe_col =
-      pipe_supported(g.nx, g.ny, fp64) && (ctx->pipe_for(g.nx, g.ny) & MSF_PIPE_COL);
+  const bool pipe_col = !fp64 || (pipe_supported(g.nx, g.ny, true) &&
+                                  (ctx->pipe_for(g.nx, g.ny) & MSF_PIPE_COL));
   alignas(64) unsigned char col_map[128];
-  if (pipe_col) MSF_CUDA(encode_column_map(psi.p, B, g.nx, g.ny, col_map, fp64));
+  if (pipe_col) MSF_CUDA(encode_col_map(fp64, psi.p, B, g, col_map));
   PassArgs row, col;
   // columns the band limit removes entirely are skipped (same grid, hence
   // the same mask, for every snapshot)
@@ -144,7 +144,7 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
   MSF_TRY(ctx->twiddles(g.ny, fp64, &row.tw));
-  MSF_TRY(ctx->twiddles(g.nx, fp64, &col.tw));
+  MSF_TRY(ctx->col_twiddles(g.nx, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.first_scale = g.nxny / g.s;
   const SegmentPlan seg_acc = segment_plan(A, partial.as<double>());
@@ -190,10 +190,7 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
         MSF_CUDA(launch_row(fp64, op, row, st));
         col.px = pbase + prop_stride * sl;
         col.py = pbase + prop_stride * sl + cbytes * g.nx;
-        if (pipe_col)
-          MSF_CUDA(launch_col_slice_pipe(col, sl + 1 == S, col_map, d_err.as<int>(), st, fp64));
-        else
-          MSF_CUDA(launch_col(fp64, sl + 1 == S ? COL_SLICE_LAST : COL_SLICE, col, st));
+        MSF_CUDA(launch_col_slice(fp64, pipe_col, sl + 1 == S, col, col_map, d_err.as<int>(), st));
       }
       SplitK sk;
       if (!fp64) {

@@ -188,7 +188,7 @@ extern "C" msf_status msf_probe_noalloc(const msf_grid* grid, const msf_optics* 
   NOALLOC_CUDA(msf::launch_row(true, msf::ROW_INV, a, s));
   a.tw = twx;
   a.scale = 1.0 / sq;
-  NOALLOC_CUDA(msf::launch_col(true, msf::COL_INV, a, s));
+  NOALLOC_CUDA(msf::launch_col(msf::COL_INV, a, s));
   // norm (overwrites the accumulator) and scale, all on the device
   NOALLOC_CUDA(msf::launch_norm2(probe_device, (int64_t)nx * ny, norm, s));
   const int64_t n = (int64_t)nx * ny;
