@@ -667,7 +667,7 @@ int64_t raster_plan_bytes(const msf_specimen* spec, bool fp64, int64_t n_probes,
   if (!fp64) b += 8 * plane * spec->n_slices + 16 * plane;   // vacuum tables
   b += 8 * n_probes + 3 * 4 * plane;                         // shifts, segments
   b += 2 * 8 * n_probes * (int64_t)(spec->g.nx + 1);         // sums (n_seg <= nx + 1)
-  if (pix_modes) b += 2 * 8 * plane;
+  if (pix_modes) b += 2 * 8 * plane + 4 * 8 * (int64_t)(spec->g.nx + 1);  // sums, ring means
   return b;
 }
 
@@ -782,22 +782,20 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
   // segments: ring bins (FEM) then the ADF detector annulus
   if (P->fem) P->rings = rings_for(ctx, g, det->dr);
   P->n_k = P->fem ? P->rings->n_k : 0;
-  std::vector<int32_t> seg_idx, seg_start{0};
-  if (P->fem) {
-    seg_idx = P->rings->pix;
+  // (pixel lists laid one after the other: rings, annulus, correlograph cells)
+  std::vector<int32_t> seg_start{0};
+  if (P->fem)
     for (int k = 0; k < P->n_k; ++k) seg_start.push_back(P->rings->start[k + 1]);
-  }
-  const std::vector<int32_t> adf_pix =
-      detector_pixels(g, det->det_inner / g.lambda, det->det_outer / g.lambda);
-  seg_idx.insert(seg_idx.end(), adf_pix.begin(), adf_pix.end());
-  seg_start.push_back((int32_t)seg_idx.size());
+  const int32_t ring_pixels = seg_start.back();
+  const PixelRuns adf = detector_runs(g, det->det_inner / g.lambda, det->det_outer / g.lambda);
+  seg_start.push_back(ring_pixels + adf.offset.back());
   P->n_seg = P->n_k + 1;
+  Cells cells;
   if (P->fem && (det->outputs & MSF_OUT_CORRELOGRAPH)) {
     // correlograph cells (k bin, phi bin) after the ADF annulus
-    const Cells cells = make_cells(g, *P->rings);
+    cells = make_cells(g, *P->rings);
     const size_t n_cells = (size_t)P->n_k * cells.n_phi;
-    const int32_t base = (int32_t)seg_idx.size();
-    seg_idx.insert(seg_idx.end(), cells.pix.begin(), cells.pix.end());
+    const int32_t base = seg_start.back();
     for (size_t c = 0; c < n_cells; ++c) seg_start.push_back(base + cells.start[c + 1]);
     P->n_seg += (int)n_cells;
   }
@@ -811,7 +809,22 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
   seg_chunk.push_back((int32_t)chunk_begin.size());
   P->n_chunks = (int)chunk_begin.size();
   chunk_begin.push_back(seg_start[P->n_seg]);
-  MSF_TRY(upload(ctx, &P->seg_idx, seg_idx));
+  MSF_TRY(ctx->alloc(&P->seg_idx, sizeof(int32_t) * std::max(1, seg_start.back())));
+  if (ring_pixels > 0)
+    MSF_CUDA(cudaMemcpyAsync(P->seg_idx.p, P->rings->pix.data(), sizeof(int32_t) * ring_pixels,
+                             cudaMemcpyHostToDevice, ctx->stream));
+  DevBuf run_base, run_offset;
+  MSF_TRY(upload(ctx, &run_base, adf.base));
+  MSF_TRY(upload(ctx, &run_offset, adf.offset));
+  MSF_CUDA(launch_expand_runs(run_base.as<int32_t>(), run_offset.as<int32_t>(),
+                              (int)adf.base.size(), P->seg_idx.as<int32_t>() + ring_pixels,
+                              ctx->stream));
+  if (!adf.base.empty()) P->setup_launches += 1;
+  if (!cells.pix.empty())
+    MSF_CUDA(cudaMemcpyAsync(P->seg_idx.as<int32_t>() + ring_pixels + adf.offset.back(),
+                             cells.pix.data(), sizeof(int32_t) * cells.pix.size(),
+                             cudaMemcpyHostToDevice, ctx->stream));
+  ctx->h2d_bytes += (int64_t)(sizeof(int32_t) * (ring_pixels + cells.pix.size()));
   MSF_TRY(upload(ctx, &P->chunk_begin, chunk_begin));
   MSF_TRY(upload(ctx, &P->seg_chunk, seg_chunk));
   MSF_TRY(ctx->alloc(&P->amp, sizeof(double) * n_probes * P->n_seg));
@@ -821,6 +834,7 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
     MSF_TRY(ctx->alloc(&P->acc_i, sizeof(double) * plane));
     MSF_CUDA(cudaMemsetAsync(P->acc_a.p, 0, P->acc_a.bytes, ctx->stream));
     MSF_CUDA(cudaMemsetAsync(P->acc_i.p, 0, P->acc_i.bytes, ctx->stream));
+    MSF_TRY(ctx->alloc(&P->ring_means, sizeof(double) * 4 * std::max(P->n_k, 1)));
   }
   // detector MTF (adfstem.cpp:298-414): table -> 2-D, BACKWARD transform,
   // band limit applied to that real-space array (kept as the reference does
@@ -944,8 +958,13 @@ msf_status finish_raster(msf_context* ctx, const RasterPlan& P, cudaStream_t str
   // the sums land in the context's pinned staging buffer (no page faults on
   // fresh host memory, copies at the pinned rate)
   const size_t rows = (size_t)P.n_probes * P.n_seg;
-  const size_t pix = P.pix_modes ? (size_t)P.plane : 0;
-  const size_t need = sizeof(double) * (2 * rows + 2 * pix);
+  // pixel modes: the ring sums come from the device; the planes themselves
+  // only when their means are asked for
+  const bool means = P.pix_modes && P.fem;
+  const size_t n_means = means ? 4 * (size_t)P.n_k : 0;
+  const size_t pix =
+      P.pix_modes && (res->mean_amplitude || res->mean_intensity) ? (size_t)P.plane : 0;
+  const size_t need = sizeof(double) * (2 * rows + n_means + 2 * pix);
   std::lock_guard<std::mutex> lock(ctx->stage_mu);
   if (ctx->host_stage_bytes < need) {
     // freeing pinned memory can wait on the device: not during a capture
@@ -960,18 +979,34 @@ msf_status finish_raster(msf_context* ctx, const RasterPlan& P, cudaStream_t str
   }
   double* amp = ctx->host_stage;
   double* inten = amp + rows;
-  double* acc_a = P.pix_modes ? inten + rows : nullptr;
-  double* acc_i = P.pix_modes ? acc_a + pix : nullptr;
+  double* ring_means = means ? inten + rows : nullptr;
+  double* acc_a = pix ? inten + rows + n_means : nullptr;
+  double* acc_i = pix ? acc_a + pix : nullptr;
+  if (means) {
+    const Grid& g = P.spec->g;
+    SegmentPlan sp;
+    sp.idx = P.seg_idx.as<int32_t>();
+    sp.chunk_begin = P.chunk_begin.as<int32_t>();
+    sp.seg_chunk = P.seg_chunk.as<int32_t>();
+    MSF_CUDA(launch_ring_means(P.acc_a.as<double>(), P.acc_i.as<double>(), sp, P.n_k,
+                               (double)(size_t)P.n_probes, P.spec->kx.as<double>(),
+                               P.spec->ky.as<double>(), g.ny, g.lambda * g.lambda,
+                               P.optics.alpha_max * P.optics.alpha_max,
+                               P.ring_means.as<double>(), stream));
+    MSF_CUDA(cudaMemcpyAsync(ring_means, P.ring_means.p, sizeof(double) * n_means,
+                             cudaMemcpyDeviceToHost, stream));
+    ctx->d2h_bytes += (int64_t)(sizeof(double) * n_means);
+  }
   MSF_TRY(download_sums(ctx, P, stream, amp, inten, acc_a, acc_i));
   static const Rings no_rings;
   return finish_host(P.spec->g, P.rings ? *P.rings : no_rings, P.optics, P.det, P.n_probes,
-                     amp, inten, acc_a, acc_i, res);
+                     amp, inten, acc_a, acc_i, res, ring_means);
 }
 
 msf_status finish_host(const Grid& g, const Rings& rings, const msf_optics& optics,
                        const msf_detect& detect, int64_t n_probes, const double* amp,
                        const double* inten, const double* acc_a, const double* acc_i,
-                       msf_results* res) {
+                       msf_results* res, const double* ring_means) {
   const int64_t plane = (int64_t)g.nx * g.ny;
   const uint32_t fem = detect.outputs & MSF_OUT_FEM_MASK;
   const bool pix_modes = detect.outputs & (MSF_OUT_V_RE | MSF_OUT_OMEGA_VIMAGE |
@@ -982,7 +1017,7 @@ msf_status finish_host(const Grid& g, const Rings& rings, const msf_optics& opti
   if (corr) cells = make_cells(g, rings);
   const int n_phi = corr ? cells.n_phi : 0;
   const int n_seg = n_k + 1 + n_k * n_phi;
-  if (pix_modes && fem && (!acc_a || !acc_i)) {
+  if (pix_modes && fem && !ring_means && (!acc_a || !acc_i)) {
     set_error("pixel FEM modes need the per-pixel sums");
     return MSF_ERR_ARG;
   }
@@ -1064,26 +1099,36 @@ msf_status finish_host(const Grid& g, const Rings& rings, const msf_optics& opti
     }
   }
   if (pix_modes) {  // adfstem.cpp:2926-3612
-    std::vector<double> mean_a(plane), mean_sq(plane), mean_i(plane), var(plane);
-    for (int64_t p = 0; p < plane; ++p) {
-      mean_a[p] = acc_a[p] / n_r;
-      mean_sq[p] = mean_a[p] * mean_a[p];
-      mean_i[p] = acc_i[p] / n_r;
+    if (acc_a && acc_i) {
+      if (res->mean_amplitude)
+        for (int64_t p = 0; p < plane; ++p) res->mean_amplitude[p] = acc_a[p] / n_r;
+      if (res->mean_intensity)
+        for (int64_t p = 0; p < plane; ++p) res->mean_intensity[p] = acc_i[p] / n_r;
     }
-    if (res->mean_amplitude) std::memcpy(res->mean_amplitude, mean_a.data(), plane * 8);
-    if (res->mean_intensity) std::memcpy(res->mean_intensity, mean_i.data(), plane * 8);
-    auto ring_sum = [&](const std::vector<double>& v, std::vector<double>* out) {
-      out->assign(n_k, 0.0);
-      for (int k = 0; k < n_k; ++k) {
-        double s = 0.0;
-        for (int32_t q = rings.start[k]; q < rings.start[k + 1]; ++q) s += v[rings.pix[q]];
-        (*out)[k] = inside[k] ? 0.0 : s;
+    // ring sums of the means: the device's, or the same sums here
+    std::vector<double> r1(n_k, 0.0), r2(n_k, 0.0), r3(n_k, 0.0), r4(n_k, 0.0);
+    const double lsq = g.lambda * g.lambda;
+    const double amax_sq = optics.alpha_max * optics.alpha_max;
+    for (int k = 0; k < n_k; ++k) {
+      if (inside[k]) continue;
+      if (ring_means) {
+        r1[k] = ring_means[4 * k];
+        r2[k] = ring_means[4 * k + 1];
+        r3[k] = ring_means[4 * k + 2];
+        r4[k] = ring_means[4 * k + 3];
+        continue;
       }
-    };
-    std::vector<double> r1, r2, r3;
-    ring_sum(mean_i, &r1);
-    ring_sum(mean_sq, &r2);
-    ring_sum(mean_a, &r3);
+      for (int32_t q = rings.start[k]; q < rings.start[k + 1]; ++q) {
+        const int32_t p = rings.pix[q];
+        const double mean_a = acc_a[p] / n_r, mean_i = acc_i[p] / n_r;
+        const double mean_sq = mean_a * mean_a;
+        r1[k] += mean_i;
+        r2[k] += mean_sq;
+        r3[k] += mean_a;
+        const double ksqr = std::pow(g.kx[p / g.ny], 2) + std::pow(g.ky[p % g.ny], 2);
+        r4[k] += lsq * ksqr <= amax_sq ? 0.0 : (mean_i / mean_sq) - 1.0;
+      }
+    }
     for (int k = 0; k < n_k; ++k) {
       const double c = (double)cnt[k];
       const double cc = (double)(cnt[k] * cnt[k]);
@@ -1093,20 +1138,8 @@ msf_status finish_host(const Grid& g, const Rings& rings, const msf_optics& opti
       if (res->v_rbar && (det->outputs & MSF_OUT_V_RBAR))
         res->v_rbar[k] = ((r2[k] / c) / (r3[k] * r3[k] / cc)) - 1.0;
     }
-    if (res->omega_vimage && (det->outputs & MSF_OUT_OMEGA_VIMAGE)) {
-      const double lsq = g.lambda * g.lambda;
-      const double amax_sq = optics.alpha_max * optics.alpha_max;
-      for (int i = 0; i < g.nx; ++i)
-        for (int j = 0; j < g.ny; ++j) {
-          const int64_t p = j + (int64_t)g.ny * i;
-          var[p] = (mean_i[p] / (mean_a[p] * mean_a[p])) - 1.0;
-          const double ksqr = std::pow(g.kx[i], 2) + std::pow(g.ky[j], 2);
-          if (lsq * ksqr <= amax_sq) var[p] = 0.0;
-        }
-      std::vector<double> r4;
-      ring_sum(var, &r4);
+    if (res->omega_vimage && (det->outputs & MSF_OUT_OMEGA_VIMAGE))
       for (int k = 0; k < n_k; ++k) res->omega_vimage[k] = r4[k] / cnt[k];
-    }
   }
   return MSF_OK;
 }
@@ -1399,7 +1432,8 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
     // the ring sums of the filtered waves)
     res->kernel_launches =
         P.setup_launches +
-        n_batches * (2 * S + 2 + (P.pix_modes ? 1 : 0) + (P.mtf ? 8 + (P.n_k > 0 ? 2 : 0) : 0));
+        n_batches * (2 * S + 2 + (P.pix_modes ? 1 : 0) + (P.mtf ? 8 + (P.n_k > 0 ? 2 : 0) : 0)) +
+        (P.pix_modes ? 1 : 0);  // the ring means of the finish
   }
   return MSF_OK;
 }

@@ -210,13 +210,14 @@ struct RasterPlan {
   DevBuf seg_idx, chunk_begin, seg_chunk;  // segments cut into chunks
   DevBuf amp, inten;            // [n_probes][n_seg] sums of |psi| and |psi|^2
   DevBuf acc_a, acc_i;          // [plane] sums over probes (pixel modes)
+  DevBuf ring_means;            // [n_k][4] ring sums of the pixel means (pixel FEM modes)
   bool mtf = false;             // detector MTF applied before the FEM sums
   DevBuf mtf2d;                 // [plane] complex FP64, band-limited as the reference does
   int64_t setup_launches = 0;
   int64_t device_bytes() const {
     return (int64_t)(d_shifts.bytes + probe64.bytes + psi0_tab.bytes + psi0k.bytes +
                      seg_idx.bytes + chunk_begin.bytes + seg_chunk.bytes + amp.bytes +
-                     inten.bytes + acc_a.bytes + acc_i.bytes + mtf2d.bytes);
+                     inten.bytes + acc_a.bytes + acc_i.bytes + ring_means.bytes + mtf2d.bytes);
   }
 };
 // Device bytes plan_raster will allocate (for admission by an HBM budget).
@@ -239,11 +240,13 @@ msf_status finish_raster(msf_context* ctx, const RasterPlan& plan, cudaStream_t 
                          msf_results* res);
 // The ADF image and FEM statistics from per-probe sums of a whole raster
 // (host only): amp / inten [n_probes][n_k + 1] (ring sums, then the ADF
-// annulus), acc_a / acc_i the per-pixel sums over all probes (pixel modes).
+// annulus), acc_a / acc_i the per-pixel sums over all probes (pixel modes);
+// with ring_means (launch_ring_means' sums) they are only read for the means
+// asked for in `res`.
 msf_status finish_host(const Grid& g, const Rings& rings, const msf_optics& optics,
                        const msf_detect& detect, int64_t n_probes, const double* amp,
                        const double* inten, const double* acc_a, const double* acc_i,
-                       msf_results* res);
+                       msf_results* res, const double* ring_means = nullptr);
 // The raster one probe at a time, one launch per reference step (FP64).
 msf_status run_raster_plain(msf_context* ctx, const msf_specimen* spec,
                             const msf_optics* optics, const msf_raster* raster,

@@ -271,6 +271,18 @@ struct SegmentPlan {
 cudaError_t launch_segment_sums(bool fp64, const void* psi, int64_t batch_stride,
                                 int nb, const SegmentPlan& sp, double* amp, double* inten,
                                 const SplitK& sk, cudaStream_t s);
+// idx[offset[n] + t] = base[n] + t for every run n and t < its length.
+cudaError_t launch_expand_runs(const int32_t* base, const int32_t* offset, int n_runs,
+                               int32_t* idx, cudaStream_t s);
+// Sums over each ring (segments 0 .. n_k - 1 of the plan) of the raster means
+// of the pixel FEM modes: out[4 k ..] = sum of mean |psi|^2, (mean |psi|)^2,
+// mean |psi| and of mean |psi|^2 / (mean |psi|)^2 - 1 (0 where lambda^2 k^2 <=
+// alpha_max^2), with mean = acc / n.  Each ring's pixels are added one after
+// the other in the ring's order without contraction, so the sums are those of
+// the host loop bit for bit.
+cudaError_t launch_ring_means(const double* acc_a, const double* acc_i, const SegmentPlan& sp,
+                              int n_k, double n, const double* kx, const double* ky, int ny,
+                              double lambda_sq, double amax_sq, double* out, cudaStream_t s);
 // Detection of the slots that finished their last slice in a slot batch.
 struct DetectSlot {
   const float2* psi = nullptr;         // the slot's exit wave (scattered, k-space)

@@ -250,14 +250,34 @@ Cells make_cells(const Grid& g, const Rings& r) {
   return c;
 }
 
-std::vector<int32_t> detector_pixels(const Grid& g, double k1, double k2) {
-  std::vector<int32_t> out;
-  for (int i = 0; i < g.nx; ++i)
-    for (int j = 0; j < g.ny; ++j) {
-      const double ksq = g.kx[i] * g.kx[i] + g.ky[j] * g.ky[j];
-      if (ksq > k1 && ksq <= k2) out.push_back((int32_t)(j + (int64_t)i * g.ny));
+PixelRuns detector_runs(const Grid& g, double k1, double k2) {
+  // Along a row ky*ky rises with j up to ny/2 and falls from there (rounded
+  // products and sums are monotone), so each half of the row holds one run
+  // and its ends are found by bisection on the annulus test itself.
+  PixelRuns r;
+  r.offset.push_back(0);
+  auto first = [](int lo, int hi, auto&& pred) {  // pred is false, then true
+    while (lo < hi) {
+      const int mid = lo + (hi - lo) / 2;
+      if (pred(mid)) hi = mid;
+      else lo = mid + 1;
     }
-  return out;
+    return lo;
+  };
+  const int half = g.ny / 2;
+  for (int i = 0; i < g.nx; ++i) {
+    auto ksq = [&](int j) { return g.kx[i] * g.kx[i] + g.ky[j] * g.ky[j]; };
+    const int a0 = first(0, half, [&](int j) { return ksq(j) > k1; });
+    const int a1 = first(a0, half, [&](int j) { return ksq(j) > k2; });
+    const int b0 = first(half, g.ny, [&](int j) { return ksq(j) <= k2; });
+    const int b1 = first(b0, g.ny, [&](int j) { return !(ksq(j) > k1); });
+    for (const auto& e : {std::pair<int, int>{a0, a1}, std::pair<int, int>{b0, b1}})
+      if (e.second > e.first) {
+        r.base.push_back((int32_t)(e.first + (int64_t)i * g.ny));
+        r.offset.push_back(r.offset.back() + (e.second - e.first));
+      }
+  }
+  return r;
 }
 
 std::vector<double> raster_points(double period, double origin, double spacing) {

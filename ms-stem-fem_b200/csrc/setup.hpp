@@ -95,8 +95,13 @@ Cells make_cells(const Grid& g, const Rings& r);
 std::vector<double> mtf_2d(const Grid& g, const double* mtf, const double* domain_sqr, int n,
                            double resolution);
 
-// ADF detector pixels k1 < kx*kx+ky*ky <= k2 (func.cpp:2593-2640).
-std::vector<int32_t> detector_pixels(const Grid& g, double k1, double k2);
+// ADF detector pixels k1 < kx*kx+ky*ky <= k2 (func.cpp:2593-2640), row by row
+// as runs of consecutive pixels: run n is pixels base[n] .. at list positions
+// offset[n] .. offset[n + 1] - 1.
+struct PixelRuns {
+  std::vector<int32_t> base, offset;
+};
+PixelRuns detector_runs(const Grid& g, double k1, double k2);
 
 // Raster positions (func.cpp:108-127, tem.cpp:1358-1378).
 std::vector<double> raster_points(double period, double origin, double spacing);
