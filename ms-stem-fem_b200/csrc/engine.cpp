@@ -532,15 +532,12 @@ msf_status build_probe(msf_context* ctx, const msf_specimen* spec, const msf_opt
                               ctx->stream));
   // BACKWARD transform, / sqrtNxNy (adfstem.cpp:686-732)
   MSF_TRY(fft2d_f64(ctx, g, probe64->as<double>(), 1, true, 1.0 / g.s));
-  // Ap = 1/sqrt(sum |psi|^2) (probe_wavefunction.cpp:287-315)
-  DevBuf d_sum;
-  MSF_TRY(ctx->alloc(&d_sum, sizeof(double)));
-  MSF_CUDA(launch_norm2(probe64->as<double>(), plane, d_sum.as<double>(), ctx->stream));
-  double sum = 0;
-  MSF_CUDA(cudaMemcpyAsync(&sum, d_sum.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  MSF_CUDA(cudaStreamSynchronize(ctx->stream));
-  const double ap = 1.0 / std::sqrt(sum);
-  MSF_CUDA(launch_scale(probe64->as<double>(), plane, ap, nullptr, ctx->stream));
+  // Ap = 1/sqrt(sum |psi|^2) (probe_wavefunction.cpp:287-315), on the device
+  DevBuf norm;
+  MSF_TRY(ctx->alloc(&norm, sizeof(double) * (kNormBlocks + 1)));
+  MSF_CUDA(launch_norm2_wide(probe64->as<double>(), plane, norm.as<double>() + 1,
+                             norm.as<double>(), ctx->stream));
+  MSF_CUDA(launch_scale(probe64->as<double>(), plane, 1.0, norm.as<double>(), ctx->stream));
   return MSF_OK;
 }
 
@@ -719,7 +716,7 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
 
   // probe
   MSF_TRY(build_probe(ctx, spec, optics, &P->probe64));
-  P->setup_launches = 5;
+  P->setup_launches = 6;
 
   // FP32 runs carry only the scattered part of each wave; the vacuum part
   // psi0 (the probe propagated with t = 1) is the same for every probe up to
@@ -731,11 +728,10 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
     MSF_TRY(ctx->alloc(&P->psi0_tab, 8 * plane * (size_t)S));
     MSF_TRY(ctx->alloc(&P->psi0k, 16 * plane));
     MSF_TRY(upload(ctx, &prop64, spec->hprop));
-    MSF_CUDA(cudaMemcpyAsync(P->psi0k.p, P->probe64.p, 16 * plane, cudaMemcpyDeviceToDevice,
-                             ctx->stream));
-    MSF_CUDA(launch_scale(P->psi0k.as<double>(), plane, g.nxny / g.s, nullptr, ctx->stream));
     PassArgs v;
     v.psi = P->psi0k.p;
+    v.probe = P->probe64.p;
+    v.first_scale = g.nxny / g.s;
     v.batch_stride = plane;
     v.nb = 1;
     v.nx = g.nx;
@@ -746,23 +742,15 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
     const void *tw_y = nullptr, *tw_x = nullptr;
     MSF_TRY(ctx->twiddles(g.ny, true, &tw_y));
     MSF_TRY(ctx->twiddles(g.nx, true, &tw_x));
-    P->setup_launches += 1;
     for (int s = 0; s < S; ++s) {
-      MSF_CUDA(launch_to_f32(P->psi0k.as<double>(), P->psi0_tab.as<float>() + 2 * plane * s,
-                             2 * plane, ctx->stream));
+      v.out32 = P->psi0_tab.as<float>() + 2 * plane * s;
       v.tw = tw_y;
-      MSF_CUDA(launch_row(true, ROW_FWD, v, ctx->stream));
+      MSF_CUDA(launch_row(true, s == 0 ? ROW_VACUUM_FIRST : ROW_VACUUM, v, ctx->stream));
       v.tw = tw_x;
       v.px = prop64.as<double>() + 2 * (size_t)(g.nx + g.ny) * s;
       v.py = prop64.as<double>() + 2 * (size_t)(g.nx + g.ny) * s + 2 * g.nx;
       MSF_CUDA(launch_col(s + 1 == S ? COL_SLICE_LAST : COL_SLICE, v, ctx->stream));
-      P->setup_launches += 3;
-      if (s + 1 < S) {
-        v.tw = tw_y;
-        v.scale = 1.0;
-        MSF_CUDA(launch_row(true, ROW_INV, v, ctx->stream));
-        P->setup_launches += 1;
-      }
+      P->setup_launches += 2;
     }
     // prop64 is released at the end of this scope: finish its readers first
     MSF_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1425,7 +1413,7 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   }
   {
     const int64_t n_batches = (n_probes + B - 1) / B;
-    // probe: synth, 2 transform passes, norm, scale (+ FP32 copy); per batch:
+    // probe: synth, 2 transform passes, norm (2), scale; per batch:
     // 2*S slice passes, the segment sums (chunks, totals) and (pixel modes)
     // the accumulation
     // (MTF: magnitude, 4 transform passes, multiply, scale, band limit and

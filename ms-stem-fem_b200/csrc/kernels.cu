@@ -259,6 +259,10 @@ row_kernel(const PassArgs a) {
       const int iy = (y < sy) ? y + N - sy : y - sy;
       v[m] = cscale(__ldg(prow + iy), fs);
     }
+  } else if constexpr (OP == ROW_VACUUM_FIRST) {
+    const C* prow = static_cast<const C*>(a.probe) + (int64_t)i * N;
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = cscale(prow[t + T * m], (Real)a.first_scale);
   } else if constexpr (OP == ROW_SPLIT_FIRST) {
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = C{(Real)0, (Real)0};
@@ -298,6 +302,14 @@ row_kernel(const PassArgs a) {
                      t, a.shifts[2 * b], a.shifts[2 * b + 1], (Real)a.inv_s);
     fft_line<Sh, false>(v, sm, t, tw, sync);
   } else if constexpr (OP == ROW_FWD) {
+    fft_line<Sh, false>(v, sm, t, tw, sync);
+  } else if constexpr (OP == ROW_VACUUM || OP == ROW_VACUUM_FIRST) {
+    // one pass a slice where inverse transform, rounding and forward
+    // transform took three (2048^2: 92 us of launches -> 45 us)
+    if constexpr (OP == ROW_VACUUM) fft_line<Sh, true>(v, sm, t, tw, sync);
+    float2* out = reinterpret_cast<float2*>(a.out32) + (int64_t)i * N;
+#pragma unroll
+    for (int m = 0; m < E; ++m) out[t + T * m] = make_float2((float)v[m].x, (float)v[m].y);
     fft_line<Sh, false>(v, sm, t, tw, sync);
   } else if constexpr (OP == ROW_INV) {
     fft_line<Sh, true>(v, sm, t, tw, sync);
@@ -646,15 +658,45 @@ __global__ void norm2_kernel(const double2* __restrict__ a, int64_t n, double* o
   if (threadIdx.x == 0) out[0] = red[0];
 }
 
-__global__ void scale_kernel(double2* a, int64_t n, double s) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) a[k] = make_double2(a[k].x * s, a[k].y * s);
+// Sum of a block's values in thread 0 (fixed order; 256 threads).
+__device__ __forceinline__ double block_sum(double s) {
+  __shared__ double red[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < (int)blockDim.x >> 5; ++w) s += red[w];
+  return s;
 }
 
-__global__ void to_f32_kernel(const double* __restrict__ in, float* __restrict__ out,
-                              int64_t n) {
+// One block cannot pull a plane faster than one SM: the norm of a 4096^2 probe
+// took 2.46 ms and of a 1024^2 one 0.107 ms in norm2_kernel; four blocks an SM
+// read at memory speed.
+__global__ void __launch_bounds__(256)
+norm2_partial_kernel(const double2* __restrict__ a, int64_t n, double* __restrict__ partial) {
+  double s = 0.0;
+  for (int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x; k < n; k += (int64_t)gridDim.x * 256) {
+    const double2 v = a[k];
+    s += v.x * v.x + v.y * v.y;
+  }
+  s = block_sum(s);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+
+__global__ void __launch_bounds__(256)
+norm2_total_kernel(const double* __restrict__ partial, int n, double* out) {
+  double s = 0.0;
+  for (int k = threadIdx.x; k < n; k += 256) s += partial[k];
+  s = block_sum(s);
+  if (threadIdx.x == 0) out[0] = s;
+}
+
+__global__ void scale_kernel(double2* a, int64_t n, double s,
+                             const double* __restrict__ dev_norm2) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) out[k] = (float)in[k];
+  if (dev_norm2) s = 1.0 / sqrt(*dev_norm2);
+  if (k < n) a[k] = make_double2(a[k].x * s, a[k].y * s);
 }
 
 // ------------------------------------------------------- detection -------
@@ -1119,6 +1161,9 @@ cudaError_t launch_row(bool fp64, RowOp op, const PassArgs& a, cudaStream_t s) {
       case ROW_INV: return row_dispatch<double, ROW_INV>(a, s);
       case ROW_SLICE: return row_dispatch<double, ROW_SLICE>(a, s);
       case ROW_SLICE_FIRST: return row_dispatch<double, ROW_SLICE_FIRST>(a, s);
+      case ROW_VACUUM: return row_dispatch<double, ROW_VACUUM>(a, s);
+      case ROW_VACUUM_FIRST: return row_dispatch<double, ROW_VACUUM_FIRST>(a, s);
+      default: return cudaErrorInvalidValue;
     }
   } else {
     switch (op) {
@@ -1252,13 +1297,18 @@ cudaError_t launch_norm2(const double* a, int64_t n, double* out, cudaStream_t s
   return cudaGetLastError();
 }
 
-cudaError_t launch_scale(double* a, int64_t n, double sc, const double*, cudaStream_t s) {
-  scale_kernel<<<blocks_for(n, 256), 256, 0, s>>>(reinterpret_cast<double2*>(a), n, sc);
+cudaError_t launch_norm2_wide(const double* a, int64_t n, double* partial, double* out,
+                              cudaStream_t s) {
+  const int blocks = std::min<unsigned>(blocks_for(n, 256), kNormBlocks);
+  norm2_partial_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const double2*>(a), n, partial);
+  norm2_total_kernel<<<1, 256, 0, s>>>(partial, blocks, out);
   return cudaGetLastError();
 }
 
-cudaError_t launch_to_f32(const double* in, float* out, int64_t n, cudaStream_t s) {
-  to_f32_kernel<<<blocks_for(n, 256), 256, 0, s>>>(in, out, n);
+cudaError_t launch_scale(double* a, int64_t n, double sc, const double* dev_norm2,
+                         cudaStream_t s) {
+  scale_kernel<<<blocks_for(n, 256), 256, 0, s>>>(reinterpret_cast<double2*>(a), n, sc,
+                                                  dev_norm2);
   return cudaGetLastError();
 }
 

@@ -57,6 +57,10 @@ enum RowOp : int {
   // Split-wave pass of a slot batch (FP32): every probe reads its own slice
   // tables and step from PassArgs::slots (ROW_SPLIT_FIRST or ROW_SPLIT).
   ROW_SLOTS = 6,
+  // Vacuum tables of split-wave runs (FP64 wave): iDFT, the real-space wave
+  // rounded to FP32 into PassArgs::out32, DFT; first, from probe * first_scale
+  ROW_VACUUM = 7,
+  ROW_VACUUM_FIRST = 8,
 };
 // Which fused operation a column pass (transform along x, strided) does.
 enum ColOp : int {
@@ -98,6 +102,7 @@ struct PassArgs {
   const void* probe = nullptr;    // [nx][ny] complex, normalised real space
   const int32_t* shifts = nullptr;// [nb][2] (sx, sy)
   double first_scale = 1.0;       // nx*ny/s
+  float* out32 = nullptr;         // [nx][ny] complex (ROW_VACUUM*)
   double scale = 1.0;             // ROW_INV / COL_INV
   // column mask and propagator
   const int32_t* mask_lo = nullptr;  // [ny]: keep i < lo[j] || i >= hi[j]
@@ -248,11 +253,13 @@ cudaError_t launch_probe_synth(double* out, const double* kx, const double* ky,
                                double y0, cudaStream_t s);
 // out[0] = sum |a|^2 over n complex doubles (deterministic, one block).
 cudaError_t launch_norm2(const double* a, int64_t n, double* out, cudaStream_t s);
-// a *= s (n complex doubles); s read from device memory when dev_scale.
-cudaError_t launch_scale(double* a, int64_t n, double s, const double* dev_rsqrt_of,
+// The same sum by many blocks: partial holds kNormBlocks doubles.
+constexpr int kNormBlocks = 592;
+cudaError_t launch_norm2_wide(const double* a, int64_t n, double* partial, double* out,
+                              cudaStream_t s);
+// a *= s (n complex doubles), or a *= 1 / sqrt(*dev_norm2) when given.
+cudaError_t launch_scale(double* a, int64_t n, double s, const double* dev_norm2,
                          cudaStream_t st);
-cudaError_t launch_to_f32(const double* in, float* out, int64_t n_real,
-                          cudaStream_t s);
 
 // ---- detection / FEM reductions on a batch of k-space waves ----
 // Pixel segments (FEM ring bins, then the ADF annulus), each cut into chunks
