@@ -36,12 +36,16 @@ namespace {
 // [16, 256] (measured on B200: 256 slots at 512^2 and 1024^2, 64 at 2048^2;
 // larger sets of wavefields run slower), bounded by the lane's probes and by
 // half the free memory shared among `lanes` lanes.
-int lane_slots(int want, int64_t plane, int lanes, int64_t probes) {
+int lane_slots(msf_context* ctx, int want, int64_t plane, int lanes, int64_t probes) {
   if (want > 0) return want;
+  const int64_t footprint = std::max<int64_t>(16, std::min<int64_t>(256, (2LL << 30) / (8 * plane)));
+  // wavefields that fit a block the context's pool already has need no look
+  // at the free memory (msf_context::default_batch)
+  const int64_t most = std::min(footprint, probes);
+  if (ctx->pool->has((size_t)(8 * plane * most))) return (int)std::max<int64_t>(1, most);
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   const int64_t cap = (int64_t)(0.5 * (double)free_b / std::max(1, lanes)) / (8 * plane);
-  const int64_t footprint = std::max<int64_t>(16, std::min<int64_t>(256, (2LL << 30) / (8 * plane)));
   return (int)std::max<int64_t>(1, std::min<int64_t>({cap, footprint, probes}));
 }
 
@@ -76,7 +80,7 @@ msf_status run_batch(msf_context* ctx, int n, const msf_specimen* const* specs,
   for (auto& kv : groups) {
     int64_t probes = 0;
     for (int i : kv.second) probes += jobs[i]->plan.n_probes;
-    const int b = lane_slots(slots, (int64_t)kv.first.first * kv.first.second,
+    const int b = lane_slots(ctx, slots, (int64_t)kv.first.first * kv.first.second,
                              (int)groups.size(), probes);
     lanes.push_back(std::make_unique<Lane>(ctx, kv.first.first, kv.first.second, b));
     MSF_TRY(lanes.back()->init());

@@ -103,6 +103,7 @@ msf_status msf_context_destroy(msf_context* ctx) {
   ctx->tw64.clear();
   ctx->tw32.clear();
   ctx->tw_pair.clear();
+  for (cudaEvent_t e : ctx->pass_events) cudaEventDestroy(e);
   {  // buffers released after this point free their memory directly
     std::lock_guard<std::mutex> lock(ctx->pool->m);
     ctx->pool->closed = true;

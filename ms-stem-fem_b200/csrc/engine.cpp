@@ -71,6 +71,12 @@ void* Pool::take(size_t bytes, size_t* got) {
   return p;
 }
 
+bool Pool::has(size_t bytes) {
+  std::lock_guard<std::mutex> lock(m);
+  auto it = blocks.lower_bound(bytes);
+  return it != blocks.end() && it->first <= 2 * bytes + (4u << 20);
+}
+
 std::recursive_mutex& capture_mutex() {
   static std::recursive_mutex m;
   return m;
@@ -166,6 +172,16 @@ msf_status msf_context::twiddles(int n, bool want64, const void** out) {
   }
   *out = it->second.p;
   return MSF_OK;
+}
+
+int msf_context::default_batch(int64_t block_per_wave, int64_t bytes_per_wave, int64_t probes,
+                               int most) {
+  const int64_t want = std::min<int64_t>(probes, most);
+  if (pool->has((size_t)(block_per_wave * want))) return (int)want;
+  size_t free_b = 0, total_b = 0;
+  cudaMemGetInfo(&free_b, &total_b);
+  const int64_t cap = (int64_t)(0.5 * (double)free_b) / bytes_per_wave;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(cap, want));
 }
 
 msf_status msf_context::col_twiddles(int n, const void** out) {
@@ -383,10 +399,7 @@ msf_status build_specimen(msf_context* ctx, const msf_grid* gin, const msf_atoms
 
   // band-limit mask (shared by the transmission build and the propagator)
   std::vector<int32_t> lo, hi;
-  if (!bandlimit_mask(g, g.bw_t, &lo, &hi)) {
-    set_error("band-limit mask is not an interval per column");
-    return MSF_ERR_UNSUPPORTED;
-  }
+  bandlimit_mask(g, g.bw_t, &lo, &hi);
   MSF_TRY(upload(ctx, &spec->mask_lo, lo));
   MSF_TRY(upload(ctx, &spec->mask_hi, hi));
   {
@@ -1144,14 +1157,13 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   const size_t cbytes = fp64 ? 16 : 8;
   const int S = P.S, n_seg = P.n_seg;
 
-  // batch of wavefields: the context's, the tuned one for this grid, or
-  // what half the free memory holds, at most 64
+  // batch of wavefields: the context's, the tuned one for this grid, or the
+  // default (64 with a detector MTF, whose FP64 planes come on top)
   int B = ctx->batch_for(g.nx, g.ny);
   if (B <= 0) {
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    const int64_t cap = (int64_t)(0.5 * (double)free_b) / (int64_t)(cbytes * plane);
-    B = (int)std::max<int64_t>(1, std::min<int64_t>(cap, 64));
+    const int64_t wave = (int64_t)cbytes * plane;
+    const int64_t most = P.mtf ? 64 : std::clamp<int64_t>((2LL << 30) / wave, 16, 256);
+    B = ctx->default_batch(wave, wave, n_probes, (int)most);
   }
   B = (int)std::min<int64_t>(B, n_probes);
   DevBuf psi, d_partial, mtf_psi, mtf_amp, mtf_int;
@@ -1212,14 +1224,15 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
 
   // events around the passes of the first (eager) batch: the pass times
   // reported with the results are measured inside the run itself
-  std::vector<cudaEvent_t> pass_ev;
-  bool timing_passes = false;
-  struct EventsGuard {
-    std::vector<cudaEvent_t>* v;
-    ~EventsGuard() {
-      for (cudaEvent_t e : *v) cudaEventDestroy(e);
-    }
-  } pass_ev_guard{&pass_ev};
+  std::vector<cudaEvent_t>& events = ctx->pass_events;  // begin, end, the passes'
+  bool timing_passes = false, timed_passes = false;
+  while (events.size() < 2 + 3 * (size_t)S) {
+    cudaEvent_t ev = nullptr;
+    MSF_CUDA(cudaEventCreate(&ev));
+    events.push_back(ev);
+  }
+  const cudaEvent_t ev0 = events[0], ev1 = events[1];
+  const cudaEvent_t* pass_ev = events.data() + 2;
 
   // one batch: 2*S fused passes then the reductions
   auto enqueue_batch = [&](int nb, const int32_t* shifts_dev, double* amp_out,
@@ -1281,9 +1294,6 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
     return MSF_OK;
   };
 
-  cudaEvent_t ev0, ev1;
-  MSF_CUDA(cudaEventCreate(&ev0));
-  MSF_CUDA(cudaEventCreate(&ev1));
   MSF_CUDA(cudaEventRecord(ev0, ctx->stream));
   cudaGraphExec_t graph_exec = nullptr;
   DevBuf stage_shift, stage_amp, stage_int;
@@ -1322,8 +1332,7 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
     } else {
       timing_passes = p0 == 0 && S >= 3;
       if (timing_passes) {
-        pass_ev.assign(3 * (size_t)S, nullptr);
-        for (auto& e : pass_ev) MSF_CUDA(cudaEventCreate(&e));
+        timed_passes = true;
         res->pass_batch = nb;
       }
       st = enqueue_batch(nb, P.d_shifts.as<int32_t>() + 2 * p0, P.amp.as<double>() + p0 * n_seg,
@@ -1389,13 +1398,11 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   }
   float ms = 0;
   MSF_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
-  cudaEventDestroy(ev0);
-  cudaEventDestroy(ev1);
   res->seconds_raster = 1e-3 * ms;
   res->seconds_setup = 0;
   res->probe_slices = n_probes * S;
   res->ms_row_pass = res->ms_col_pass = 0;
-  if (!pass_ev.empty()) {
+  if (timed_passes) {
     // row passes of slices 1..S-1 (after the probe-placing first), column
     // passes of slices 0..S-2 (before the last, which stops in k-space)
     double row_ms = 0, col_ms = 0;

@@ -37,6 +37,8 @@ struct Pool {
   // A cached block of at least `bytes` and at most twice that (+4 MiB), or
   // nullptr; *got receives its size.
   void* take(size_t bytes, size_t* got);
+  // Whether take() would find one.
+  bool has(size_t bytes);
   // Keeps a released block.  Waits for the device first, as cudaFree does,
   // so that no kernel still in flight on any stream can see it reused.
   void give(void* p, size_t bytes);
@@ -139,6 +141,16 @@ struct msf_context {
   };
   std::map<RingKey, std::shared_ptr<const msf::Rings>> ring_cache;
   std::mutex ring_mu;
+  // CUDA events around the passes a run times, kept for the next run
+  std::vector<cudaEvent_t> pass_events;
+  // Wavefields per launch when neither the caller nor the tuner chose: about
+  // 2 GiB of them, 16 to 256 (256 at 1024^2 FP32, where a larger launch reads
+  // the slice's tables once for more probes: 4 to 5 % faster than 64), at most
+  // `probes` and what half the free memory holds at bytes_per_wave.  A batch
+  // whose largest buffer (block_per_wave a wavefield) fits a block the pool
+  // already has needs no look at the free memory: that call takes 0.1 ms on a
+  // quiet host and has taken 74 ms on a busy one.
+  int default_batch(int64_t block_per_wave, int64_t bytes_per_wave, int64_t probes, int most);
   // pinned host buffer the per-probe and per-pixel sums of a raster are
   // copied into before the host finish (grown on demand, reused by every
   // raster; freed with the context)
@@ -274,7 +286,7 @@ msf_status run_batch(msf_context* ctx, int n, const msf_specimen* const* specs,
 cudaError_t encode_col_map(bool fp64, void* psi, int nb, const Grid& g, void* map);
 cudaError_t launch_col_slice(bool fp64, bool pipe_col, bool last, const PassArgs& a,
                              const void* map, int* err, cudaStream_t s);
-int lane_slots(int want, int64_t plane, int lanes, int64_t probes);
+int lane_slots(msf_context* ctx, int want, int64_t plane, int lanes, int64_t probes);
 // The plain FP32 split-wave row pass's L2 prefetch ahead (MSF_ROW_L2AHEAD)
 // for rows of `spec`'s grid: distance and live element ranges.
 void set_row_ahead(const msf_context* ctx, const msf_specimen* spec, PassArgs* row);

@@ -111,10 +111,8 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
   // batch: the wavefields, their FP64 average and (MTF) the filtered waves
   int B = ctx->batch_for(g.nx, g.ny);
   if (B <= 0) {
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
     const int64_t per = (int64_t)(cbytes + 16 + (A.mtf ? 16 : 0)) * plane;
-    B = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)(0.5 * (double)free_b) / per, 64));
+    B = ctx->default_batch(16 * plane, per, n_probes, 64);
   }
   B = (int)std::min<int64_t>(B, n_probes);
   int max_chunks = A.n_chunks;

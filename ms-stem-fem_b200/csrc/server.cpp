@@ -225,7 +225,7 @@ struct msf_server {
     auto it = lanes.find(key);
     if (it == lanes.end()) {
       const int64_t plane = (int64_t)r.grid.nx * r.grid.ny;
-      const int b = lane_slots(slots, plane, (int)lanes.size() + 1, 1 << 30);
+      const int b = lane_slots(ctx, slots, plane, (int)lanes.size() + 1, 1 << 30);
       // smaller grids on higher-priority streams: one step per 4x the pixels
       int least = 0, greatest = 0;
       cudaDeviceGetStreamPriorityRange(&least, &greatest);

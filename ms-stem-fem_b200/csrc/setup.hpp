@@ -54,7 +54,7 @@ bool probe_shifts(const Grid& g, const std::vector<double>& x_p,
 
 // Band-limit mask kx^2+ky^2 < bw_t^2 as, per column j, "keep i < lo[j] or
 // i >= hi[j]" (bw_limit.cpp:30-47 and slice.cpp:1385-1419 use the same set).
-bool bandlimit_mask(const Grid& g, double cutoff, std::vector<int32_t>* lo,
+void bandlimit_mask(const Grid& g, double cutoff, std::vector<int32_t>* lo,
                     std::vector<int32_t>* hi);
 
 // Propagator tables (slice.cpp:1293-1363), interleaved re/im.
