@@ -459,8 +459,9 @@ msf_status run_sharded(msf_context* ctx, const msf_specimen* spec, const msf_opt
       return MSF_ERR_CUDA;
     }
     MSF_TRY(nccl_wait(comm, "the exchange of detector rows and pixel sums"));
-    MSF_CUDA(cudaMemcpyAsync(rows_all.data(), recv.p, recv.bytes, cudaMemcpyDeviceToHost,
-                             comm->stream));
+    // the rows' own size: a pool block can be larger than what was asked for
+    MSF_CUDA(cudaMemcpyAsync(rows_all.data(), recv.p, rows_all.size() * sizeof(double),
+                             cudaMemcpyDeviceToHost, comm->stream));
     if (pix) {
       MSF_CUDA(launch_rank_sum(pix_recv.as<double>(), world, 2 * plane, pix_sum.as<double>(),
                                comm->stream));
