@@ -40,15 +40,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
-// Table entries from global or shared memory.
-struct GlobalTable {
-  const float2* p;
-  __device__ __forceinline__ float2 operator()(int k) const { return __ldg(p + k); }
-};
-struct SharedTable {
-  const float2* p;
-  __device__ __forceinline__ float2 operator()(int k) const { return p[k]; }
-};
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes,
                                          uint64_t* bar) {
   asm volatile(

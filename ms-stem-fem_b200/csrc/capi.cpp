@@ -102,7 +102,9 @@ msf_status msf_context_destroy(msf_context* ctx) {
   cudaStreamSynchronize(ctx->stream);
   ctx->tw64.clear();
   ctx->tw32.clear();
-  ctx->tw_pair.clear();
+  ctx->tw_col32.clear();
+  ctx->tw_col64.clear();
+  ctx->tw_row64.clear();
   for (cudaEvent_t e : ctx->pass_events) cudaEventDestroy(e);
   {  // buffers released after this point free their memory directly
     std::lock_guard<std::mutex> lock(ctx->pool->m);

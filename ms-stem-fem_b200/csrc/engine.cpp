@@ -184,33 +184,31 @@ int msf_context::default_batch(int64_t block_per_wave, int64_t bytes_per_wave, i
   return (int)std::max<int64_t>(1, std::min<int64_t>(cap, want));
 }
 
-msf_status msf_context::col_twiddles(int n, const void** out) {
-  if (fp64) return twiddles(n, true, out);
-  auto it = tw_pair.find(n);
-  if (it == tw_pair.end()) {
-    std::vector<float> f;
-    fill_pair_twiddles(n, f);
+msf_status msf_context::slice_twiddles(bool f64, int nx, int ny, const void** row,
+                                       const void** col) {
+  auto table = [&](std::map<int, DevBuf>& m, int n, auto&& fill) -> msf_status {
+    if (m.count(n)) return MSF_OK;
     DevBuf b;
-    MSF_TRY(upload(this, &b, f));
-    it = tw_pair.emplace(n, std::move(b)).first;
+    MSF_TRY(upload(this, &b, fill()));
+    m.emplace(n, std::move(b));
+    return MSF_OK;
+  };
+  if (f64) {
+    std::vector<double> h;
+    MSF_TRY(table(tw_row64, ny, [&]() -> auto& { fill_row64_twiddles(ny, h); return h; }));
+    MSF_TRY(table(tw_col64, nx, [&]() -> auto& { fill_col_twiddles(nx, h); return h; }));
+    *row = tw_row64.at(ny).p;
+    *col = tw_col64.at(nx).p;
+  } else {
+    std::vector<float> h;
+    MSF_TRY(twiddles(ny, false, row));
+    MSF_TRY(table(tw_col32, nx, [&]() -> auto& { fill_col_twiddles(nx, h); return h; }));
+    *col = tw_col32.at(nx).p;
   }
-  *out = it->second.p;
   return MSF_OK;
 }
 
 namespace msf {
-
-cudaError_t encode_col_map(bool fp64, void* psi, int nb, const Grid& g, void* map) {
-  return fp64 ? encode_column_map(psi, nb, g.nx, g.ny, map)
-              : encode_pair_map(psi, nb, g.nx, g.ny, map);
-}
-
-cudaError_t launch_col_slice(bool fp64, bool pipe_col, bool last, const PassArgs& a,
-                             const void* map, int* err, cudaStream_t s) {
-  if (!fp64) return launch_col_pair(a, last, map, err, s);
-  return pipe_col ? launch_col_slice_pipe(a, last, map, err, s)
-                  : launch_col(last ? COL_SLICE_LAST : COL_SLICE, a, s);
-}
 
 namespace {
 
@@ -407,32 +405,38 @@ msf_status build_specimen(msf_context* ctx, const msf_grid* gin, const msf_atoms
     std::vector<uint8_t> dead(g.ny);
     for (int j = 0; j < g.ny; ++j) dead[j] = lo[j] == 0 && hi[j] == g.nx;
     spec->n_live_columns = (int)std::count(dead.begin(), dead.end(), 0);
-    const bool fp = ctx->fp64;
-    const int T = row_line_threads(g.ny, fp), cols = fp ? pipe_cols_for(g.nx) : col_pair_tile(g.nx);
-    if (T > 0 && g.ny / T <= 32 && cols > 0 && spec->n_live_columns < g.ny) {
+    // per layout: bit m of word t, column t + T m, and the live column groups
+    auto bits_of = [&](int T) {
       std::vector<uint32_t> bits(T, 0u);
       for (int t = 0; t < T; ++t)
         for (int m = 0; m < g.ny / T; ++m)
           if (dead[t + T * m]) bits[t] |= 1u << m;
+      return bits;
+    };
+    auto groups_of = [&](int cols) {
       std::vector<int32_t> groups;
-      for (int gi = 0; gi < g.ny / cols; ++gi) {
-        bool live = false;
-        for (int c = 0; c < cols; ++c) live = live || !dead[gi * cols + c];
-        if (live) groups.push_back(gi);
+      for (int gi = 0; gi < g.ny / cols; ++gi)
+        if (std::find(dead.begin() + gi * cols, dead.begin() + (gi + 1) * cols, 0) !=
+            dead.begin() + (gi + 1) * cols)
+          groups.push_back(gi);
+      return groups;
+    };
+    if (spec->n_live_columns < g.ny) {
+      const bool fp = ctx->fp64;
+      spec->h_dead_bits = bits_of(fp ? row64_threads(g.ny) : row_line_threads(g.ny));
+      spec->h_live_groups = groups_of(col_tile(g.nx, fp));
+      spec->n_live_groups = (int)spec->h_live_groups.size();
+      MSF_TRY(upload(ctx, &spec->dead_bits, spec->h_dead_bits));
+      MSF_TRY(upload(ctx, &spec->live_groups, spec->h_live_groups));
+      if (!fp) {
+        const std::vector<int32_t> vac = groups_of(col_tile(g.nx, true));
+        spec->n_vac_live_groups = (int)vac.size();
+        MSF_TRY(upload(ctx, &spec->vac_dead_bits, bits_of(row64_threads(g.ny))));
+        MSF_TRY(upload(ctx, &spec->vac_live_groups, vac));
+        // the same bits for the row pass's alternative schedule
+        const int T1 = staged_row_threads(g.ny, 1);
+        if (T1 > 0) MSF_TRY(upload(ctx, &spec->dead_bits_alt, bits_of(T1)));
       }
-      MSF_TRY(upload(ctx, &spec->dead_bits, bits));
-      MSF_TRY(upload(ctx, &spec->live_groups, groups));
-      const int T1 = fp ? 0 : staged_row_threads(g.ny, 1);
-      if (T1 > 0) {  // the same bits for the staged row pass's schedule 1
-        std::vector<uint32_t> bits1(T1, 0u);
-        for (int t = 0; t < T1; ++t)
-          for (int m = 0; m < g.ny / T1; ++m)
-            if (dead[t + T1 * m]) bits1[t] |= 1u << m;
-        MSF_TRY(upload(ctx, &spec->dead_bits_alt, bits1));
-      }
-      spec->n_live_groups = (int)groups.size();
-      spec->h_dead_bits = bits;
-      spec->h_live_groups = groups;
     }
     // live element ranges of a row: [0, d0) and [d1, ny) around one run of
     // removed columns [d0, d1), widened to even bounds
@@ -591,8 +595,7 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
   row.nb = col.nb = nb;
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
-  MSF_TRY(ctx->twiddles(g.ny, fp64, &row.tw));
-  MSF_TRY(ctx->col_twiddles(g.nx, &col.tw));
+  MSF_TRY(ctx->slice_twiddles(fp64, g.nx, g.ny, &row.tw, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.trans = spec->t.p;
   row.psi0 = psi0.p;
@@ -607,14 +610,12 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
   const int row_sched = !fp64 && staged_row_supported(g.nx, g.ny) && (pipe & MSF_ROW_ALT) ? 1 : 0;
   const bool pipe_row = !fp64 && !staged_row && !row_sched && pipe_supported(g.nx, g.ny) &&
                         (pipe & MSF_PIPE_ROW);
-  const bool pipe_col =
-      !fp64 || (pipe_supported(g.nx, g.ny, true) && (pipe & MSF_PIPE_COL));
   alignas(64) unsigned char col_map[128];
   DevBuf d_err;
   MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), ctx->stream));
-  if (pipe_col) MSF_CUDA(encode_col_map(fp64, psi.p, nb, g, col_map));
-  if (pipe_col && !pipe_row && spec->n_live_groups > 0) {  // skip removed columns
+  MSF_CUDA(encode_col_map(fp64, psi.p, nb, g.nx, g.ny, col_map));
+  if (!pipe_row && spec->n_live_groups > 0) {  // skip removed columns
     row.row_dead_bits = spec->dead_bits.as<uint32_t>();
     row.row_dead_io = 3;  // a slice between the first and the last
     col.live_groups = spec->live_groups.as<int32_t>();
@@ -632,10 +633,11 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
                                                       row_sched)
            : row_sched == 1 ? launch_row_split_alt(row_staged, ctx->stream)
            : pipe_row       ? launch_row_split_pipe(row, d_err.as<int>(), ctx->stream)
-                            : launch_row(fp64, rop, row, ctx->stream);
+           : fp64           ? launch_row64(rop, row, ctx->stream)
+                            : launch_row(false, rop, row, ctx->stream);
   };
   auto col_pass = [&]() {
-    return launch_col_slice(fp64, pipe_col, false, col, col_map, d_err.as<int>(), ctx->stream);
+    return launch_col_slice(fp64, false, col, col_map, d_err.as<int>(), ctx->stream);
   };
   std::vector<cudaEvent_t> ev(2 * reps + 2);
   for (auto& e : ev) MSF_CUDA(cudaEventCreate(&e));
@@ -753,20 +755,37 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
     v.mask_hi = spec->mask_hi.as<int32_t>();
     v.inv_s = 1.0 / (g.s * g.s);  // Q(1, psi) = psi/s, then FFT2 and /s
     const void *tw_y = nullptr, *tw_x = nullptr;
-    MSF_TRY(ctx->twiddles(g.ny, true, &tw_y));
-    MSF_TRY(ctx->twiddles(g.nx, true, &tw_x));
+    MSF_TRY(ctx->slice_twiddles(true, g.nx, g.ny, &tw_y, &tw_x));
+    if (spec->n_vac_live_groups > 0) {
+      v.row_dead_bits = spec->vac_dead_bits.as<uint32_t>();
+      v.live_groups = spec->vac_live_groups.as<int32_t>();
+      v.n_live_groups = spec->n_vac_live_groups;
+    }
+    alignas(64) unsigned char map[128];
+    MSF_CUDA(encode_col_map(true, P->psi0k.p, 1, g.nx, g.ny, map));
+    DevBuf d_err;
+    MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
+    MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), ctx->stream));
     for (int s = 0; s < S; ++s) {
       v.out32 = P->psi0_tab.as<float>() + 2 * plane * s;
+      v.row_dead_io = (s > 0 ? 1 : 0) | (s + 1 < S ? 2 : 0);
       v.tw = tw_y;
-      MSF_CUDA(launch_row(true, s == 0 ? ROW_VACUUM_FIRST : ROW_VACUUM, v, ctx->stream));
+      MSF_CUDA(launch_row64(s == 0 ? ROW_VACUUM_FIRST : ROW_VACUUM, v, ctx->stream));
       v.tw = tw_x;
       v.px = prop64.as<double>() + 2 * (size_t)(g.nx + g.ny) * s;
       v.py = prop64.as<double>() + 2 * (size_t)(g.nx + g.ny) * s + 2 * g.nx;
-      MSF_CUDA(launch_col(s + 1 == S ? COL_SLICE_LAST : COL_SLICE, v, ctx->stream));
+      MSF_CUDA(launch_col_slice(true, s + 1 == S, v, map, d_err.as<int>(), ctx->stream));
       P->setup_launches += 2;
     }
+    int err_flag = 0;
+    MSF_CUDA(cudaMemcpyAsync(&err_flag, d_err.p, sizeof(int), cudaMemcpyDeviceToHost,
+                             ctx->stream));
     // prop64 is released at the end of this scope: finish its readers first
     MSF_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (err_flag) {
+      set_error("a vacuum column pass gave up waiting for a tile copy (bounded wait)");
+      return MSF_ERR_TIMEOUT;
+    }
   }
 
   // per-probe pixel shifts: the reference's search carries its position
@@ -1188,16 +1207,14 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   const int row_sched = !fp64 && staged_row_supported(g.nx, g.ny) && (pipe & MSF_ROW_ALT) ? 1 : 0;
   const bool pipe_row = !fp64 && !staged_row && !row_sched && pipe_supported(g.nx, g.ny) &&
                         (pipe & MSF_PIPE_ROW);
-  const bool pipe_col =
-      !fp64 || (pipe_supported(g.nx, g.ny, true) && (pipe & MSF_PIPE_COL));
   alignas(64) unsigned char col_map[128];
   DevBuf d_err;
   MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), ctx->stream));
-  if (pipe_col) MSF_CUDA(encode_col_map(fp64, psi.p, B, g, col_map));
+  MSF_CUDA(encode_col_map(fp64, psi.p, B, g.nx, g.ny, col_map));
 
   PassArgs row, col;
-  if (pipe_col && !pipe_row && spec->n_live_groups > 0) {  // skip removed columns
+  if (!pipe_row && spec->n_live_groups > 0) {  // skip removed columns
     row.row_dead_bits = spec->dead_bits.as<uint32_t>();
     col.live_groups = spec->live_groups.as<int32_t>();
     col.n_live_groups = spec->n_live_groups;
@@ -1206,8 +1223,7 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   row.batch_stride = col.batch_stride = plane;
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
-  MSF_TRY(ctx->twiddles(g.ny, fp64, &row.tw));
-  MSF_TRY(ctx->col_twiddles(g.nx, &col.tw));
+  MSF_TRY(ctx->slice_twiddles(fp64, g.nx, g.ny, &row.tw, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.prefetch_tables = (!fp64 && (pipe & MSF_ROW_PREFETCH)) ? 1 : 0;
   if (!fp64 && !staged_row && row_sched == 0 && !pipe_row && (pipe & MSF_ROW_L2AHEAD))
@@ -1262,13 +1278,14 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
       }
       else if (pipe_row && op == ROW_SPLIT)
         MSF_CUDA(launch_row_split_pipe(row, d_err.as<int>(), ctx->stream));
+      else if (fp64)
+        MSF_CUDA(launch_row64(op, row, ctx->stream));
       else
-        MSF_CUDA(launch_row(fp64, op, row, ctx->stream));
+        MSF_CUDA(launch_row(false, op, row, ctx->stream));
       if (timing_passes) MSF_CUDA(cudaEventRecord(pass_ev[3 * s + 1], ctx->stream));
       col.px = pbase + prop_stride * s;
       col.py = pbase + prop_stride * s + cbytes * g.nx;
-      MSF_CUDA(launch_col_slice(fp64, pipe_col, s + 1 == S, col, col_map, d_err.as<int>(),
-                                ctx->stream));
+      MSF_CUDA(launch_col_slice(fp64, s + 1 == S, col, col_map, d_err.as<int>(), ctx->stream));
       if (timing_passes) MSF_CUDA(cudaEventRecord(pass_ev[3 * s + 2], ctx->stream));
     }
     SplitK sk;

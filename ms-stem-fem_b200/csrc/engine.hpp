@@ -107,8 +107,9 @@ struct msf_context {
   int64_t allocated() const { return pool->live; }
   int64_t h2d_bytes = 0, d2h_bytes = 0;
   cudaStream_t stream = nullptr;
-  // twiddle tables per length; tw_pair: the FP32 column pass's (fft_pair.cuh)
-  std::map<int, msf::DevBuf> tw64, tw32, tw_pair;
+  // twiddle tables per length; tw_col32, tw_col64: the column slice pass's,
+  // tw_row64: the FP64 row slice pass's (fft_lines.cuh)
+  std::map<int, msf::DevBuf> tw64, tw32, tw_col32, tw_col64, tw_row64;
   // autotuned launch tiling per grid (nx, ny): probes per launch and the
   // pipelined-pass mask (msf_tune, or imported wisdom)
   struct Tuned {
@@ -162,8 +163,8 @@ struct msf_context {
   bool keep_potentials = false;
   msf_status alloc(msf::DevBuf* b, size_t bytes);
   msf_status twiddles(int n, bool fp64, const void** out);
-  // the table of the context's column slice pass
-  msf_status col_twiddles(int n, const void** out);
+  // the tables of the slice passes of one precision
+  msf_status slice_twiddles(bool fp64, int nx, int ny, const void** row, const void** col);
 };
 
 struct msf_specimen {
@@ -181,6 +182,9 @@ struct msf_specimen {
   // the row-pass zero bits in the layout of the alternative FFT schedule of
   // the staged row pass (FP32 contexts; empty when it does not apply)
   msf::DevBuf dead_bits_alt;
+  // FP32 contexts: the same for the FP64 passes that build vacuum tables
+  msf::DevBuf vac_dead_bits, vac_live_groups;
+  int n_vac_live_groups = 0;
   std::vector<uint32_t> h_dead_bits;  // host copies (slot lanes compare them)
   std::vector<int32_t> h_live_groups;
   int n_live_groups = 0, n_live_columns = 0;
@@ -281,11 +285,6 @@ msf_status time_passes(msf_context* ctx, const msf_specimen* spec, int nb, int r
 msf_status run_batch(msf_context* ctx, int n, const msf_specimen* const* specs,
                      const msf_optics* optics, const msf_raster* rasters,
                      const msf_detect* detects, msf_results* results, int slots);
-// The tensor map and launch of the context's batched column slice pass: FP32
-// contexts always, FP64 ones when `pipe_col` (else the plain kernel, no map).
-cudaError_t encode_col_map(bool fp64, void* psi, int nb, const Grid& g, void* map);
-cudaError_t launch_col_slice(bool fp64, bool pipe_col, bool last, const PassArgs& a,
-                             const void* map, int* err, cudaStream_t s);
 int lane_slots(msf_context* ctx, int want, int64_t plane, int lanes, int64_t probes);
 // The plain FP32 split-wave row pass's L2 prefetch ahead (MSF_ROW_L2AHEAD)
 // for rows of `spec`'s grid: distance and live element ranges.

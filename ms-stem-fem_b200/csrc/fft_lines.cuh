@@ -1,0 +1,409 @@
+// Two FP32 lines, or one FP64 line, per thread: the Stockham FFT of the column
+// passes and of the FP64 row pass.
+//
+// A thread holds E elements.  In FP32 an element is a Pair, the same element of
+// two lines with both real parts in one register pair and both imaginary parts
+// in another, so that every operation is one packed instruction (FADD2 / FMUL2 /
+// FFMA2) and twiddles and propagators are loaded once for the two lines.
+//
+// A radix-R stage after NS-point sub-transforms computes
+//   X[k + NS m] = sum_r v[r] W_(NS R)^(r (k + NS m))
+// by log2 R decimation-in-time layers: the layer of block size B pairs m and
+// m + B/2 with the twiddle W_(NS B)^(k + NS m), so the stage's own twiddles
+// cost nothing beyond the butterflies' (a separate multiply before an
+// untwiddled DFT costs one more complex product an element).  A butterfly is
+//   r = a + w b (four FMAs),  q = 2 a - r (two),
+// six instead of the four multiplies and four adds of product, sum and
+// difference.  m >= B/4 needs no twiddle of its own: it is -i times that of
+// m - B/4.  A stage of radix 32 then reads 16 twiddles per thread and two
+// lines where the product form reads 31 per line.
+#pragma once
+#include <cmath>
+#include <vector>
+
+#include "fft_core.cuh"
+
+namespace msf {
+
+struct Pair {
+  float2 re, im;  // .x the first line, .y the second
+};
+
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 f2neg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 f2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 f2sub(float2 a, float2 b) { return __fadd2_rn(a, f2neg(b)); }
+__device__ __forceinline__ float2 f2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// Columns (rows) the band limit always removes: it keeps |k| < N/3 of the
+// N-point line, so of the E slots (slot m holds elements T m .. T m + T - 1)
+// those from ceil(E / 3) to E - ceil(E / 3) - 1 hold removed elements only.
+template <int E> __host__ __device__ constexpr int dead_lo() { return (E + 2) / 3; }
+template <int E> __host__ __device__ constexpr int dead_hi() { return E - (E + 2) / 3; }
+template <int E> __host__ __device__ constexpr bool dead_slot(int m) {
+  return m >= dead_lo<E>() && m < dead_hi<E>();
+}
+
+// An N-point schedule: E elements of each line per thread, T threads, radices
+// R0 R1 [R2].
+template <int N_, int E_, int R0_, int R1_, int R2_ = 1> struct LineShape {
+  static constexpr int N = N_, E = E_, S = R2_ > 1 ? 3 : 2, T = N_ / E_;
+  static_assert(R0_ * R1_ * R2_ == N_);
+  __host__ __device__ static constexpr int radix(int s) {
+    return s == 0 ? R0_ : s == 1 ? R1_ : R2_;
+  }
+  __host__ __device__ static constexpr int ns(int s) {
+    return s == 0 ? 1 : s == 1 ? R0_ : R0_ * R1_;
+  }
+  // entries of one butterfly's twiddles: one for B = 2 and 4, B/4 after
+  __host__ __device__ static constexpr int tw_rows(int r) {
+    return r <= 2 ? r / 2 : r == 4 ? 2 : tw_rows(r / 2) + r / 4;
+  }
+  // stage s >= 1's table [row][k], k < ns(s), after the earlier stages'
+  __host__ __device__ static constexpr int tw_off(int s) {
+    return s <= 1 ? 0 : tw_off(s - 1) + tw_rows(radix(s - 1)) * ns(s - 1);
+  }
+};
+// columns: the fewest stages
+template <int N> struct ColShapeOf;
+template <> struct ColShapeOf<64> { using type = LineShape<64, 8, 8, 8>; };
+template <> struct ColShapeOf<128> { using type = LineShape<128, 16, 16, 8>; };
+template <> struct ColShapeOf<256> { using type = LineShape<256, 16, 16, 16>; };
+template <> struct ColShapeOf<512> { using type = LineShape<512, 32, 32, 16>; };
+template <> struct ColShapeOf<1024> { using type = LineShape<1024, 32, 32, 32>; };
+template <> struct ColShapeOf<2048> { using type = LineShape<2048, 32, 32, 8, 8>; };
+template <> struct ColShapeOf<4096> { using type = LineShape<4096, 32, 32, 32, 4>; };
+template <int N> using ColShape = typename ColShapeOf<N>::type;
+// FP64 rows: the same up to 1024 points; beyond, where 32 elements a thread
+// spill, 16 (2048: 40 us a probe against 59)
+template <int N> struct RowShapeOf { using type = ColShape<N>; };
+template <> struct RowShapeOf<2048> { using type = LineShape<2048, 16, 16, 16, 8>; };
+template <> struct RowShapeOf<4096> { using type = LineShape<4096, 16, 16, 16, 16>; };
+template <int N> using RowShape = typename RowShapeOf<N>::type;
+
+// A shape's twiddles w_(NS B)^(k + NS m), stage by stage in the order the
+// layers read them, (cos, -sin) pairs computed in FP64.
+template <class Sh, typename Real> void line_twiddles(std::vector<Real>& out) {
+  const double two_pi = 6.283185307179586476925286766559;
+  for (int s = 1; s < Sh::S; ++s)
+    for (int B = 2; B <= Sh::radix(s); B *= 2)
+      for (int m = 0; m < (B > 4 ? B / 4 : 1); ++m)
+        for (int k = 0; k < Sh::ns(s); ++k) {
+          const double x = two_pi * (k + (double)Sh::ns(s) * m) / ((double)Sh::ns(s) * B);
+          out.push_back((Real)std::cos(x));
+          out.push_back((Real)-std::sin(x));
+        }
+}
+
+// Table entries from global or shared memory.
+template <typename C> struct GlobalTable {
+  using type = C;
+  const C* p;
+  __device__ __forceinline__ C operator()(int k) const { return __ldg(p + k); }
+};
+template <typename C> struct SharedTable {
+  using type = C;
+  const C* p;
+  __device__ __forceinline__ C operator()(int k) const { return p[k]; }
+};
+
+// What a thread holds per element: a Pair (two FP32 lines) or a double2 (one
+// FP64 line), 16 bytes either way, so both share the kernels' layouts.
+template <class V> struct LineOf;
+template <> struct LineOf<Pair> {
+  using Real = float;
+  using C = float2;     // a table entry
+  using Half = float2;  // both lines' real or imaginary parts
+  using Mem = float4;
+};
+template <> struct LineOf<double2> {
+  using Real = double;
+  using C = double2;
+  using Half = double;
+  using Mem = double2;
+};
+__device__ __forceinline__ void put(float4* p, const Pair& v) {
+  *p = make_float4(v.re.x, v.re.y, v.im.x, v.im.y);
+}
+__device__ __forceinline__ void get(const float4* p, Pair& v) {
+  const float4 x = *p;
+  v = Pair{make_float2(x.x, x.y), make_float2(x.z, x.w)};
+}
+__device__ __forceinline__ void put(double2* p, const double2& v) { *p = v; }
+__device__ __forceinline__ void get(const double2* p, double2& v) { v = *p; }
+// two adjacent complex values in memory (re, im, re, im), or one FP64 one
+__device__ __forceinline__ void put_cols(float4* p, const Pair& v) {
+  *p = make_float4(v.re.x, v.im.x, v.re.y, v.im.y);
+}
+__device__ __forceinline__ void get_cols(const float4* p, Pair& v) {
+  const float4 x = *p;
+  v = Pair{make_float2(x.x, x.z), make_float2(x.y, x.w)};
+}
+__device__ __forceinline__ void put_cols(double2* p, const double2& v) { *p = v; }
+__device__ __forceinline__ void get_cols(const double2* p, double2& v) { v = *p; }
+__device__ __forceinline__ float2& re_of(Pair& v) { return v.re; }
+__device__ __forceinline__ float2& im_of(Pair& v) { return v.im; }
+__device__ __forceinline__ double& re_of(double2& v) { return v.x; }
+__device__ __forceinline__ double& im_of(double2& v) { return v.y; }
+__device__ __forceinline__ Pair vneg(const Pair& b) { return Pair{f2neg(b.re), f2neg(b.im)}; }
+__device__ __forceinline__ double2 vneg(const double2& b) { return make_double2(-b.x, -b.y); }
+template <class V> __device__ __forceinline__ V vzero();
+template <> __device__ __forceinline__ Pair vzero<Pair>() { return Pair{f2(0.f), f2(0.f)}; }
+template <> __device__ __forceinline__ double2 vzero<double2>() { return make_double2(0.0, 0.0); }
+
+// a, b <- a + w b, a - w b, with w = c + i s (its conjugate when INV);
+// NEED: bit 0 the sum is used, bit 1 the difference
+template <bool INV, int NEED = 3>
+__device__ __forceinline__ void bfly(Pair& a, Pair& b, float c, float s) {
+  const float2 C = f2(c), S = f2(INV ? -s : s);
+  if constexpr (NEED & 1) {
+    Pair r;
+    r.re = f2fma(f2neg(S), b.im, f2fma(C, b.re, a.re));
+    r.im = f2fma(S, b.re, f2fma(C, b.im, a.im));
+    if constexpr (NEED & 2) {
+      b.re = f2fma(f2(2.f), a.re, f2neg(r.re));
+      b.im = f2fma(f2(2.f), a.im, f2neg(r.im));
+    }
+    a = r;
+  } else if constexpr (NEED & 2) {
+    Pair q;
+    q.re = f2fma(S, b.im, f2fma(f2neg(C), b.re, a.re));
+    q.im = f2fma(f2neg(S), b.re, f2fma(f2neg(C), b.im, a.im));
+    b = q;
+  }
+}
+// w = 1
+__device__ __forceinline__ void bfly_1(Pair& a, Pair& b) {
+  const Pair r{f2add(a.re, b.re), f2add(a.im, b.im)};
+  b = Pair{f2sub(a.re, b.re), f2sub(a.im, b.im)};
+  a = r;
+}
+// w = -i (forward) or +i (inverse)
+template <bool INV>
+__device__ __forceinline__ void bfly_i(Pair& a, Pair& b) {
+  Pair r, q;
+  if constexpr (INV) {
+    r = Pair{f2sub(a.re, b.im), f2add(a.im, b.re)};
+    q = Pair{f2add(a.re, b.im), f2sub(a.im, b.re)};
+  } else {
+    r = Pair{f2add(a.re, b.im), f2sub(a.im, b.re)};
+    q = Pair{f2sub(a.re, b.im), f2add(a.im, b.re)};
+  }
+  a = r;
+  b = q;
+}
+
+template <bool INV, int NEED = 3>
+__device__ __forceinline__ void bfly(double2& a, double2& b, double c, double s0) {
+  const double s = INV ? -s0 : s0;
+  if constexpr (NEED & 1) {
+    const double2 r = make_double2(fma(-s, b.y, fma(c, b.x, a.x)), fma(s, b.x, fma(c, b.y, a.y)));
+    if constexpr (NEED & 2) b = make_double2(fma(2.0, a.x, -r.x), fma(2.0, a.y, -r.y));
+    a = r;
+  } else if constexpr (NEED & 2) {
+    b = make_double2(fma(s, b.y, fma(-c, b.x, a.x)), fma(-s, b.x, fma(-c, b.y, a.y)));
+  }
+}
+__device__ __forceinline__ void bfly_1(double2& a, double2& b) {
+  const double2 r = cadd(a, b);
+  b = csub(a, b);
+  a = r;
+}
+template <bool INV>
+__device__ __forceinline__ void bfly_i(double2& a, double2& b) {
+  const double2 w = INV ? make_double2(-b.y, b.x) : make_double2(b.y, -b.x);
+  const double2 r = cadd(a, w);
+  b = csub(a, w);
+  a = r;
+}
+
+// Layers B, 2B, .. R of a stage's butterfly over u[0..R) (bit-reversed in,
+// natural out).  k: this butterfly's first entry of the table tw, rows NS apart.
+// ZIN: E slots' dead range is zero on entry (first layer of the first stage,
+// slot of u[bitrev(r)] = r, R = E); ZOUT: not needed on exit (last layer).
+template <int R, int B, int NS, bool INV, bool ZIN, bool ZOUT, int NB, int BI, class V, class Tw>
+__device__ __forceinline__ void line_layers(V (&u)[R], const Tw& tw, int k) {
+  if constexpr (B <= R) {
+    constexpr int H = B / 2;
+    constexpr int ROWS = H >= 2 ? H / 2 : 1;  // twiddles of this layer
+    constexpr int ROW0 = B == 2 ? 0 : B == 4 ? 1 : B / 4;
+    typename Tw::type w[ROWS];
+    if constexpr (NS > 1) {
+#pragma unroll
+      for (int m = 0; m < ROWS; ++m) w[m] = tw(k + (ROW0 + m) * NS);
+    }
+    sfor<0, R, B>([&](auto baseI) {
+      sfor<0, H>([&](auto mI) {
+        constexpr int base = decltype(baseI)::value, m = decltype(mI)::value;
+        V& a = u[base + m];
+        V& b = u[base + m + H];
+        if constexpr (NS == 1) {
+          if constexpr (ZIN && B == 2) {
+            constexpr int ra = bitrev(base, ilog2(R)), rb = bitrev(base + 1, ilog2(R));
+            if constexpr (dead_slot<R>(ra) && dead_slot<R>(rb)) {
+            } else if constexpr (dead_slot<R>(rb)) {
+              b = a;
+            } else if constexpr (dead_slot<R>(ra)) {
+              a = b;
+              b = vneg(b);
+            } else {
+              bfly_1(a, b);
+            }
+          } else if constexpr (m == 0) {
+            bfly_1(a, b);
+          } else if constexpr (4 * m == B) {
+            bfly_i<INV>(a, b);
+          } else {
+            using Real = typename LineOf<V>::Real;
+            constexpr Real c = (Real)cos64(m * (64 / B)), s = (Real)-sin64(m * (64 / B));
+            bfly<INV>(a, b, c, s);
+          }
+        } else {
+          // outputs of the last layer: element slots BI + NB m
+          constexpr int E = R * NB;
+          constexpr int need = !(ZOUT && B == R) ? 3
+                               : (dead_slot<E>(BI + NB * m) ? 0 : 1) |
+                                     (dead_slot<E>(BI + NB * (m + H)) ? 0 : 2);
+          if constexpr (m < ROWS) bfly<INV, need>(a, b, w[m].x, w[m].y);
+          else bfly<INV, need>(a, b, w[m - ROWS].y, -w[m - ROWS].x);  // -i w
+        }
+      });
+    });
+    line_layers<R, 2 * B, NS, INV, ZIN, ZOUT, NB, BI>(u, tw, k);
+  }
+}
+
+// Exchange slot of element a of a line: the low three bits are XORed
+// with those of the stage-0 thread that writes it, so that the eight lanes of
+// a 16-byte access phase hit eight different slots both in the stride-R0
+// writes of the first exchange and in the unit-stride accesses of all others
+// (whose lanes share a / R0 mod 8), with no padding: the buffer is exactly
+// the line, and a column tile can be exchanged in place.
+template <class Sh> __device__ __forceinline__ int line_slot(int a) {
+  return a ^ ((a >> ilog2(Sh::radix(0))) & 7);
+}
+
+struct NoHook {
+  __device__ __forceinline__ void operator()() const {}
+};
+
+// Transforms the thread's elements in place; v[m] holds element t + T m on
+// entry and on exit.  at(a): where exchanged element a of this line lies in
+// shared memory; tw: the shape's table; sync: a barrier over the T threads of
+// the line, which must have passed one since they last read the buffer; hook:
+// run once the buffer has been read for the last time.
+template <class Sh, bool INV, bool ZIN, bool ZOUT, class V, class Tw, class At, class Sync,
+          class Hook = NoHook>
+__device__ __forceinline__ void fft_lines(V (&v)[Sh::E], int t, const Tw& tw, At&& at,
+                                         Sync&& sync, Hook&& hook = Hook{}) {
+  constexpr int N = Sh::N, E = Sh::E, T = Sh::T;
+  sfor<0, Sh::S>([&](auto sI) {
+    constexpr int s = decltype(sI)::value;
+    constexpr int R = Sh::radix(s), NB = E / R, NS = Sh::ns(s);
+    if constexpr (s > 0) {
+      sfor<0, NB>([&](auto bI) {
+        constexpr int b = decltype(bI)::value;
+        const int j = t + T * b;
+        sfor<0, R>([&](auto rI) {
+          constexpr int r = decltype(rI)::value;
+          get(at(j + r * (N / R)), v[b + r * NB]);
+        });
+      });
+      if constexpr (s + 1 == Sh::S) hook();
+      else sync();
+    }
+    sfor<0, NB>([&](auto bI) {
+      constexpr int b = decltype(bI)::value;
+      const int k = (t + T * b) & (NS - 1);
+      V u[R];
+      sfor<0, R>([&](auto rI) {
+        constexpr int r = decltype(rI)::value;
+        u[bitrev(r, ilog2(R))] = v[b + r * NB];
+      });
+      line_layers<R, 2, NS, INV, ZIN && s == 0 && R == E, ZOUT && s + 1 == Sh::S, NB, b>(
+          u, tw, Sh::tw_off(s) + k);
+      sfor<0, R>([&](auto rI) {
+        constexpr int r = decltype(rI)::value;
+        v[b + r * NB] = u[r];
+      });
+    });
+    if constexpr (s + 1 < Sh::S) {
+      sfor<0, NB>([&](auto bI) {
+        constexpr int b = decltype(bI)::value;
+        const int j = t + T * b;
+        const int base = (j / NS) * NS * R + (j & (NS - 1));
+        sfor<0, R>([&](auto rI) {
+          constexpr int r = decltype(rI)::value;
+          put(at(base + r * NS), v[b + r * NB]);
+        });
+      });
+      sync();
+    }
+  });
+}
+
+// The same transform with the exchanges in two halves (real parts, then
+// imaginary parts) through a buffer of 8 bytes an element: half the shared
+// memory for two more barriers.  x(a): where exchanged element a of this line
+// lies; start: the barrier that ends the buffer's previous use (a no-op when
+// the caller has passed one); after: run once, after the first barrier.
+template <class Sh, bool INV, bool ZIN, bool ZOUT, class V, class Tw, class X, class Sync,
+          class Start, class After>
+__device__ __forceinline__ void fft_lines_split(V (&v)[Sh::E], int t, const Tw& tw, X&& x,
+                                               Sync&& sync, Start&& start, After&& after) {
+  constexpr int N = Sh::N, E = Sh::E, T = Sh::T;
+  sfor<0, Sh::S>([&](auto sI) {
+    constexpr int s = decltype(sI)::value;
+    constexpr int R = Sh::radix(s), NB = E / R, NS = Sh::ns(s);
+    sfor<0, NB>([&](auto bI) {
+      constexpr int b = decltype(bI)::value;
+      const int k = (t + T * b) & (NS - 1);
+      V u[R];
+      sfor<0, R>([&](auto rI) {
+        constexpr int r = decltype(rI)::value;
+        u[bitrev(r, ilog2(R))] = v[b + r * NB];
+      });
+      line_layers<R, 2, NS, INV, ZIN && s == 0 && R == E, ZOUT && s + 1 == Sh::S, NB, b>(
+          u, tw, Sh::tw_off(s) + k);
+      sfor<0, R>([&](auto rI) {
+        constexpr int r = decltype(rI)::value;
+        v[b + r * NB] = u[r];
+      });
+    });
+    if constexpr (s + 1 < Sh::S) {
+      constexpr int R2 = Sh::radix(s + 1), NB2 = E / R2;
+      sfor<0, 2>([&](auto hI) {
+        constexpr int h = decltype(hI)::value;
+        if constexpr (s == 0 && h == 0) start();
+        else sync();
+        sfor<0, NB>([&](auto bI) {
+          constexpr int b = decltype(bI)::value;
+          const int j = t + T * b;
+          const int base = (j / NS) * NS * R + (j & (NS - 1));
+          sfor<0, R>([&](auto rI) {
+            constexpr int r = decltype(rI)::value;
+            *x(base + r * NS) = h == 0 ? re_of(v[b + r * NB]) : im_of(v[b + r * NB]);
+          });
+        });
+        sync();
+        if constexpr (s == 0 && h == 0) after();
+        typename LineOf<V>::Half w[E];
+        sfor<0, NB2>([&](auto bI) {
+          constexpr int b = decltype(bI)::value;
+          sfor<0, R2>([&](auto rI) {
+            constexpr int r = decltype(rI)::value;
+            w[b + r * NB2] = *x(t + T * b + r * (N / R2));
+          });
+        });
+        sfor<0, E>([&](auto mI) {
+          constexpr int m = decltype(mI)::value;
+          if constexpr (h == 0) re_of(v[m]) = w[m];
+          else im_of(v[m]) = w[m];
+        });
+      });
+    }
+  });
+}
+
+}  // namespace msf

@@ -8,11 +8,13 @@
 //   row pass    (contiguous, along y):  iDFT_y, t * psi / s (quirk kept),
 //                                       DFT_y                  [ROW_SLICE]
 //   column pass (strided,   along x):   DFT_x, / s, band-limit mask,
-//                                       propagator, iDFT_x     [COL_SLICE]
+//                                       propagator, iDFT_x     [column kernels]
 // which together equal the reference's iFFT2 -> *t -> FFT2 -> bw_limit ->
 // propagate (adfstem.cpp:1891-2048).  The first slice's row pass reads the
 // shifted probe directly (ROW_SLICE_FIRST, adfstem.cpp:1632-1837) and the
-// last slice's column pass stops in k-space for detection (COL_SLICE_LAST).
+// last slice's column pass stops in k-space for detection.  The column passes
+// and the FP64 row passes are built in their own files; here are the FP32 row
+// pass and the full 2-D transforms of the set-up in both precisions.
 #include "kernels.h"
 #include "fft_core.cuh"
 
@@ -28,7 +30,7 @@ namespace {
 constexpr double kRefPi = 3.14159265369;  // the reference's PI (adfstem.hpp:55)
 constexpr int kSmemBudget = 220 * 1024;
 
-// FP64 row passes: CTAs of 64 threads, four to an SM at up to 255
+// FP64 set-up row transforms: CTAs of 64 threads, four to an SM at up to 255
 // registers, so their load and transform phases run out of step (measured
 // 17 % faster at 1024^2 and 9 % at 2048^2 than one 256-thread CTA per SM).
 #ifndef MSF_ROW_THREADS
@@ -248,31 +250,16 @@ row_kernel(const PassArgs a) {
     }
     return;
   }
-  if constexpr (OP == ROW_SLICE_FIRST) {
-    const int sx = a.shifts[2 * b], sy = a.shifts[2 * b + 1];
-    const int ix = (i < sx) ? i + a.nx - sx : i - sx;
-    const C* prow = static_cast<const C*>(a.probe) + (int64_t)ix * N;
-    const Real fs = (Real)a.first_scale;
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-      const int y = t + T * m;
-      const int iy = (y < sy) ? y + N - sy : y - sy;
-      v[m] = cscale(__ldg(prow + iy), fs);
-    }
-  } else if constexpr (OP == ROW_VACUUM_FIRST) {
-    const C* prow = static_cast<const C*>(a.probe) + (int64_t)i * N;
-#pragma unroll
-    for (int m = 0; m < E; ++m) v[m] = cscale(prow[t + T * m], (Real)a.first_scale);
-  } else if constexpr (OP == ROW_SPLIT_FIRST) {
+  if constexpr (OP == ROW_SPLIT_FIRST) {
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = C{(Real)0, (Real)0};
-  } else if constexpr (OP == ROW_SPLIT || OP == ROW_SLICE) {
+  } else if constexpr (OP == ROW_SPLIT) {
     // columns removed by the band limit were not stored: they are zero
     const uint32_t skip = (a.row_dead_bits && (a.row_dead_io & 1)) ? __ldg(a.row_dead_bits + t)
                                                                   : 0u;
-    if (OP == ROW_SPLIT && a.l2_ahead > 0)
+    if (a.l2_ahead > 0)
       prefetch_rows_ahead<C, N, LINES>(a, by_probe);
-    if (OP == ROW_SPLIT && a.prefetch_tables) {
+    if (a.prefetch_tables) {
 #pragma unroll
       for (int m = 0; m < E; ++m)
         v[m] = ((skip >> m) & 1u) ? C{(Real)0, (Real)0} : ld_stream(row + t + T * m);
@@ -303,37 +290,13 @@ row_kernel(const PassArgs a) {
     fft_line<Sh, false>(v, sm, t, tw, sync);
   } else if constexpr (OP == ROW_FWD) {
     fft_line<Sh, false>(v, sm, t, tw, sync);
-  } else if constexpr (OP == ROW_VACUUM || OP == ROW_VACUUM_FIRST) {
-    // one pass a slice where inverse transform, rounding and forward
-    // transform took three (2048^2: 92 us of launches -> 45 us)
-    if constexpr (OP == ROW_VACUUM) fft_line<Sh, true>(v, sm, t, tw, sync);
-    float2* out = reinterpret_cast<float2*>(a.out32) + (int64_t)i * N;
-#pragma unroll
-    for (int m = 0; m < E; ++m) out[t + T * m] = make_float2((float)v[m].x, (float)v[m].y);
-    fft_line<Sh, false>(v, sm, t, tw, sync);
-  } else if constexpr (OP == ROW_INV) {
+  } else {  // ROW_INV
     fft_line<Sh, true>(v, sm, t, tw, sync);
     const Real s = (Real)a.scale;
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = cscale(v[m], s);
-  } else {
-    if constexpr (OP == ROW_SLICE) fft_line<Sh, true>(v, sm, t, tw, sync);
-    // transmission multiply with the reference's in-place update order
-    // (adfstem.cpp:1929-1949): the new real part feeds the imaginary part.
-    const C* trow = static_cast<const C*>(a.trans) + (int64_t)i * N;
-    const Real is = (Real)a.inv_s;
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-      if (m % kLoadChunk == 0) load_fence();
-      const C tv = __ldg(trow + t + T * m);
-      const Real re = (tv.x * v[m].x - tv.y * v[m].y) * is;
-      const Real im = (tv.x * v[m].y + tv.y * re) * is;
-      v[m] = C{re, im};
-    }
-    fft_line<Sh, false>(v, sm, t, tw, sync);
   }
-  if constexpr (OP == ROW_SLICE || OP == ROW_SLICE_FIRST || OP == ROW_SPLIT ||
-                OP == ROW_SPLIT_FIRST) {
+  if constexpr (OP == ROW_SPLIT || OP == ROW_SPLIT_FIRST) {
     if (a.row_dead_bits) {  // columns the next band limit removes entirely
       const uint32_t dead = __ldg(a.row_dead_bits + t);
       if (a.row_dead_io & 2) {  // nobody reads them: leave them unstored
@@ -383,30 +346,12 @@ col_kernel(const PassArgs a) {
     fft_line<Sh, false>(v, sm, t, tw, sync);
     if constexpr (OP != COL_FWD) {
       const int lo = __ldg(a.mask_lo + j), hi = __ldg(a.mask_hi + j);
-      if constexpr (OP == COL_FWD_MASK_INV) {
 #pragma unroll
-        for (int m = 0; m < E; ++m) {
-          const int i = t + T * m;
-          if (!(i < lo || i >= hi)) v[m] = C{(Real)0, (Real)0};
-        }
-      } else {
-        const Real is = (Real)a.inv_s;
-        const C pyj = __ldg(static_cast<const C*>(a.py) + j);
-        const C* px = static_cast<const C*>(a.px);
-#pragma unroll
-        for (int m = 0; m < E; ++m) {
-          if (m % kLoadChunk == 0) load_fence();
-          const int i = t + T * m;
-          if (i < lo || i >= hi) {
-            const C p = cmul(__ldg(px + i), pyj);  // slice.cpp:1396-1412
-            v[m] = cmul(p, cscale(v[m], is));
-          } else {
-            v[m] = C{(Real)0, (Real)0};
-          }
-        }
+      for (int m = 0; m < E; ++m) {
+        const int i = t + T * m;
+        if (!(i < lo || i >= hi)) v[m] = C{(Real)0, (Real)0};
       }
-      if constexpr (OP == COL_FWD_MASK_INV || OP == COL_SLICE)
-        fft_line<Sh, true>(v, sm, t, tw, sync);
+      fft_line<Sh, true>(v, sm, t, tw, sync);
     }
   }
 #pragma unroll
@@ -1141,15 +1086,15 @@ bool supported_length(int n) {
   return n == 64 || n == 128 || n == 256 || n == 512 || n == 1024 || n == 2048 || n == 4096;
 }
 
-int row_line_threads(int n, bool fp64) {
+int row_line_threads(int n) {
   switch (n) {
-    case 64: return fp64 ? Shape<64, double>::T : Shape<64, float>::T;
-    case 128: return fp64 ? Shape<128, double>::T : Shape<128, float>::T;
-    case 256: return fp64 ? Shape<256, double>::T : Shape<256, float>::T;
-    case 512: return fp64 ? Shape<512, double>::T : Shape<512, float>::T;
-    case 1024: return fp64 ? Shape<1024, double>::T : Shape<1024, float>::T;
-    case 2048: return fp64 ? Shape<2048, double>::T : Shape<2048, float>::T;
-    case 4096: return fp64 ? Shape<4096, double>::T : Shape<4096, float>::T;
+    case 64: return Shape<64, float>::T;
+    case 128: return Shape<128, float>::T;
+    case 256: return Shape<256, float>::T;
+    case 512: return Shape<512, float>::T;
+    case 1024: return Shape<1024, float>::T;
+    case 2048: return Shape<2048, float>::T;
+    case 4096: return Shape<4096, float>::T;
   }
   return 0;
 }
@@ -1159,23 +1104,15 @@ cudaError_t launch_row(bool fp64, RowOp op, const PassArgs& a, cudaStream_t s) {
     switch (op) {
       case ROW_FWD: return row_dispatch<double, ROW_FWD>(a, s);
       case ROW_INV: return row_dispatch<double, ROW_INV>(a, s);
-      case ROW_SLICE: return row_dispatch<double, ROW_SLICE>(a, s);
-      case ROW_SLICE_FIRST: return row_dispatch<double, ROW_SLICE_FIRST>(a, s);
-      case ROW_VACUUM: return row_dispatch<double, ROW_VACUUM>(a, s);
-      case ROW_VACUUM_FIRST: return row_dispatch<double, ROW_VACUUM_FIRST>(a, s);
-      default: return cudaErrorInvalidValue;
-    }
-  } else {
-    switch (op) {
-      case ROW_SLICE: return row_dispatch<float, ROW_SLICE>(a, s);
-      case ROW_SLICE_FIRST: return row_dispatch<float, ROW_SLICE_FIRST>(a, s);
-      case ROW_SPLIT: return row_dispatch<float, ROW_SPLIT>(a, s);
-      case ROW_SPLIT_FIRST: return row_dispatch<float, ROW_SPLIT_FIRST>(a, s);
-      case ROW_SLOTS: return row_dispatch<float, ROW_SLOTS>(a, s);
-      default: return cudaErrorInvalidValue;  // set-up transforms run in FP64
+      default: return cudaErrorInvalidValue;  // the slice loop's: launch_row64
     }
   }
-  return cudaErrorInvalidValue;
+  switch (op) {
+    case ROW_SPLIT: return row_dispatch<float, ROW_SPLIT>(a, s);
+    case ROW_SPLIT_FIRST: return row_dispatch<float, ROW_SPLIT_FIRST>(a, s);
+    case ROW_SLOTS: return row_dispatch<float, ROW_SLOTS>(a, s);
+    default: return cudaErrorInvalidValue;  // set-up transforms run in FP64
+  }
 }
 
 cudaError_t launch_row_split_alt(const PassArgs& a, cudaStream_t s) {
@@ -1193,8 +1130,6 @@ cudaError_t launch_col(ColOp op, const PassArgs& a, cudaStream_t s) {
     case COL_FWD: return col_dispatch<double, COL_FWD>(a, s);
     case COL_INV: return col_dispatch<double, COL_INV>(a, s);
     case COL_FWD_MASK_INV: return col_dispatch<double, COL_FWD_MASK_INV>(a, s);
-    case COL_SLICE: return col_dispatch<double, COL_SLICE>(a, s);
-    case COL_SLICE_LAST: return col_dispatch<double, COL_SLICE_LAST>(a, s);
   }
   return cudaErrorInvalidValue;
 }

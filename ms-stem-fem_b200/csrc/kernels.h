@@ -46,6 +46,7 @@ inline cudaError_t smem_limit_once(const void* func, int bytes, PerDevice& once)
 enum RowOp : int {
   ROW_FWD = 0,          // forward DFT along y
   ROW_INV = 1,          // inverse DFT along y, then * scale
+  // FP64 slice passes (launch_row64)
   ROW_SLICE = 2,        // inverse DFT, transmission multiply, forward DFT
   ROW_SLICE_FIRST = 3,  // place shifted probe, transmission multiply, fwd DFT
   // Split-wave slice passes (FP32): the buffer holds only the scattered part
@@ -57,7 +58,7 @@ enum RowOp : int {
   // Split-wave pass of a slot batch (FP32): every probe reads its own slice
   // tables and step from PassArgs::slots (ROW_SPLIT_FIRST or ROW_SPLIT).
   ROW_SLOTS = 6,
-  // Vacuum tables of split-wave runs (FP64 wave): iDFT, the real-space wave
+  // Vacuum tables of split-wave runs (FP64 wave, launch_row64): iDFT, the real-space wave
   // rounded to FP32 into PassArgs::out32, DFT; first, from probe * first_scale
   ROW_VACUUM = 7,
   ROW_VACUUM_FIRST = 8,
@@ -67,8 +68,6 @@ enum ColOp : int {
   COL_FWD = 0,           // forward DFT along x
   COL_INV = 1,           // inverse DFT along x, then * scale
   COL_FWD_MASK_INV = 2,  // forward DFT, band-limit mask, inverse DFT
-  COL_SLICE = 3,         // fwd DFT, /s, mask, propagator, inverse DFT
-  COL_SLICE_LAST = 4,    // fwd DFT, /s, mask, propagator (stay in k-space)
 };
 
 // One probe slot's step in a slot batch: probes of different specimens (of
@@ -160,10 +159,10 @@ struct SplitK {
 
 // Returns false if the length is not supported.
 bool supported_length(int n);
-// Threads per line of the row transform of length n (its T); 0 if unsupported.
-int row_line_threads(int n, bool fp64);
-// Columns per tile of the pipelined FP64 column pass (0 if unsupported).
-int pipe_cols_for(int nx);
+// Threads per line of the FP32 row transform of length n (its T); 0 if
+// unsupported.
+int row_line_threads(int n);
+// FP64: the set-up transforms ROW_FWD and ROW_INV; FP32: the split-wave ops.
 cudaError_t launch_row(bool fp64, RowOp op, const PassArgs& a, cudaStream_t s);
 // CTAs of the FP32 split-wave row pass (ROW_SPLIT, default schedule) that
 // the current device holds at once for rows of length ny (0 if
@@ -174,12 +173,18 @@ int row_split_resident_ctas(int ny);
 // in that schedule's layout, staged_row_threads(ny, 1)); row lengths
 // 256..2048.
 cudaError_t launch_row_split_alt(const PassArgs& a, cudaStream_t s);
-cudaError_t launch_col(ColOp op, const PassArgs& a, cudaStream_t s);  // FP64
+// FP64 set-up transforms: COL_FWD, COL_INV, COL_FWD_MASK_INV.
+cudaError_t launch_col(ColOp op, const PassArgs& a, cudaStream_t s);
 
-// ---- persistent TMA-pipelined slice passes (kernels_pipe.cu) ----
-// The FP64 column pass: grids with sides 256..1024; the split-wave row pass
-// (FP32 only): 256..2048.
-bool pipe_supported(int nx, int ny, bool fp64 = false);
+// ---- FP64 row passes of the slice loop (kernels_row64.cu) ----
+// ROW_SLICE, ROW_SLICE_FIRST, ROW_VACUUM, ROW_VACUUM_FIRST; a.tw from
+// fill_row64_twiddles, row_dead_bits in row64_threads' layout.
+cudaError_t launch_row64(RowOp op, const PassArgs& a, cudaStream_t s);
+int row64_threads(int ny);
+void fill_row64_twiddles(int n, std::vector<double>& out);
+
+// ---- variants of the FP32 row pass (kernels_pipe.cu), sides 256..2048 ----
+bool pipe_supported(int nx, int ny);
 // Split-wave row pass for slices after the first; *err set to 1 if a copy
 // never arrived (bounded wait).
 cudaError_t launch_row_split_pipe(const PassArgs& a, int* err, cudaStream_t s);
@@ -198,24 +203,19 @@ bool staged_row_supported(int nx, int ny);
 int staged_row_threads(int ny, int schedule);
 cudaError_t launch_row_split_staged(const PassArgs& a, int* err, cudaStream_t s,
                                     int schedule = 0);
-// FP64 column slice pass (COL_SLICE, or COL_SLICE_LAST when `last`);
-// `tensor_map` from encode_column_map over the same batch buffer.
-cudaError_t launch_col_slice_pipe(const PassArgs& a, bool last, const void* tensor_map,
-                                  int* err, cudaStream_t s);
-// Encode the 2-D tensor map (128 bytes) the FP64 column pass loads tiles with.
-cudaError_t encode_column_map(void* psi, int nb, int nx, int ny, void* map_out);
-
-// ---- the FP32 column pass (kernels_col32.cu), sides 64..4096 ----
-// COL_SLICE, or COL_SLICE_LAST when `last`, or per slot when a.slots is set;
-// a.tw from fill_pair_twiddles, `tensor_map` (128 bytes) from encode_pair_map
-// over the same batch buffer; *err set to 1 if a copy never arrived (bounded
-// wait).  The columns of a live group: col_pair_tile(nx) neighbours.
-cudaError_t launch_col_pair(const PassArgs& a, bool last, const void* tensor_map, int* err,
-                            cudaStream_t s);
-int col_pair_tile(int nx);  // 0 if unsupported
-cudaError_t encode_pair_map(void* psi, int nb, int nx, int ny, void* map_out);
-// Twiddles of the packed transform of length n, stage by stage (fft_pair.cuh).
-void fill_pair_twiddles(int n, std::vector<float>& out);
+// ---- the column slice pass (kernels_col.cu), sides 64..4096 ----
+// Up to the next slice, or stopping in k-space when `last`, or per slot when
+// a.slots is set (FP32); a.tw from fill_col_twiddles, `tensor_map` (128 bytes)
+// from encode_col_map over the same batch buffer; *err set to 1 if a copy never
+// arrived (bounded wait).  A live group is col_tile(nx, fp64) neighbouring
+// columns.
+cudaError_t launch_col_slice(bool fp64, bool last, const PassArgs& a, const void* tensor_map,
+                             int* err, cudaStream_t s);
+int col_tile(int nx, bool fp64);  // 0 if unsupported
+cudaError_t encode_col_map(bool fp64, void* psi, int nb, int nx, int ny, void* map_out);
+// Twiddles of the packed transform of length n, stage by stage (fft_lines.cuh).
+void fill_col_twiddles(int n, std::vector<float>& out);
+void fill_col_twiddles(int n, std::vector<double>& out);
 
 // Twiddle table e^{-2 pi i m / n}, m < n, computed in FP64 on the host.
 void fill_twiddles(int n, double* host_interleaved /* 2n */);

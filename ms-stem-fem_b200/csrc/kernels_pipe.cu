@@ -1,14 +1,10 @@
-// Persistent, TMA-pipelined slice passes: the FP64 column pass and variants
-// of the FP32 split-wave row pass.
+// Variants of the FP32 split-wave row pass with asynchronous copies.
 //
-// One CTA per SM walks a list of work items (a group of rows, or a group of
-// columns, of one probe).  While it transforms item k out of one shared
-// buffer, the tensor-memory accelerator already copies item k+1 into the
-// other: rows arrive as 1-D bulk copies (cp.async.bulk), column tiles as
-// 2-D tiled copies through a tensor map (cp.async.bulk.tensor), both
-// completing on an mbarrier.  The transform itself is the same register
-// Stockham FFT as kernels.cu; the buffer that just delivered the item also
-// serves as the exchange buffer.
+// The pipelined pass: one CTA per SM walks a list of row groups of one probe.
+// While it transforms item k out of one shared buffer, bulk copies
+// (cp.async.bulk, completing on an mbarrier) already bring item k+1 into the
+// other.  The transform is the register Stockham FFT of kernels.cu; the buffer
+// that just delivered the item also serves as the exchange buffer.
 //
 // Every wait is bounded: if an mbarrier phase does not complete within
 // kSpinLimit polls the CTA records an error in *err and leaves its loop,
@@ -247,130 +243,8 @@ row_split_staged_kernel(const PassArgs a, int* err) {
   for (int m = 0; m < E; ++m) row[t + T * m] = v[m];
 }
 
-// ----------------------------------------------------- column slice pass --
-// Resident CTAs per SM the register allocator must allow: at least
-// MSF_COL_PIPE_THREADS_PER_SM threads of the pass per SM.
-#ifndef MSF_COL_PIPE_THREADS_PER_SM
-#define MSF_COL_PIPE_THREADS_PER_SM 256
-#endif
-constexpr int col_pipe_min_ctas(int threads) {
-  return threads >= MSF_COL_PIPE_THREADS_PER_SM ? 1 : MSF_COL_PIPE_THREADS_PER_SM / threads;
-}
-
-// FP64 runs (a complex value is two 8-byte tensor-map elements); the FP32
-// column pass is kernels_col32.cu.
-template <typename Real, int N, int COLS, bool LAST>
-__global__ void __launch_bounds__(COLS * Shape<N, Real>::T,
-                                  col_pipe_min_ctas(COLS * Shape<N, Real>::T))
-col_slice_pipe_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap, int* err) {
-  using C = Cx<Real>;
-  using Sh = Shape<N, Real>;
-  using SM = Smem<Sh, (int)sizeof(C), COLS, true>;
-  constexpr int E = Sh::E, T = Sh::T;
-  constexpr int EPC = (int)sizeof(C) / 8;  // tensor-map elements per complex value
-  constexpr int BOX = N < 256 ? N : 256;
-  constexpr int RAW = (N * COLS > COLS * SM::stride ? N * COLS : COLS * SM::stride);
-  constexpr int BUF = (RAW + 15) / 16 * 16;  // 128-byte multiple
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  C* bufs = reinterpret_cast<C*>(smem_raw);
-  __shared__ uint64_t bars[2];
-  __shared__ int flag;
-  const int c = threadIdx.x % COLS, t = threadIdx.x / COLS;
-  // column groups to walk: all, or those with any column the band limit
-  // keeps (the row pass stored zeros in the others)
-  const int groups = a.live_groups ? a.n_live_groups : a.ny / COLS;
-  const int items = a.nb * groups;
-  auto group_of = [&](int gi) { return a.live_groups ? __ldg(a.live_groups + gi) : gi; };
-  auto sync = [] { __syncthreads(); };
-  auto issue = [&](int item, int which) {
-    const int gi = item / a.nb, b = item - gi * a.nb;
-    const int g = group_of(gi);
-    C* dst = bufs + which * BUF;
-    mbar_expect_tx(&bars[which], N * COLS * (int)sizeof(C));
-#pragma unroll
-    for (int q = 0; q < N / BOX; ++q)
-      tile_g2s(dst + q * BOX * COLS, &tmap, g * COLS * EPC, b * a.nx + q * BOX, &bars[which]);
-  };
-  if (threadIdx.x == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  int item = blockIdx.x;
-  if (threadIdx.x == 0) {
-    if (item < items) issue(item, 0);
-    if (item + (int)gridDim.x < items) issue(item + gridDim.x, 1);
-  }
-  uint32_t parity[2] = {0, 0};
-  const C* tw = static_cast<const C*>(a.tw);
-  const Real is = (Real)a.inv_s;
-  const C* px = static_cast<const C*>(a.px);
-  int k = 0;
-  for (; item < items; ++k, item += gridDim.x) {
-    const int w = k & 1;
-    if (!cta_wait(&bars[w], parity[w], &flag)) {
-      if (threadIdx.x == 0) {
-        atomicExch(err, 1);
-        if (item + (int)gridDim.x < items) mbar_wait_bounded(&bars[w ^ 1], parity[w ^ 1]);
-      }
-      return;
-    }
-    parity[w] ^= 1;
-    const int gi = item / a.nb, b = item - gi * a.nb;
-    const int g = group_of(gi);
-    const int j = g * COLS + c;
-    {
-      C* base = bufs + w * BUF;
-      C v[E];
-#pragma unroll
-      for (int m = 0; m < E; ++m) v[m] = base[(t + T * m) * COLS + c];
-      // the transform's first exchange opens with a barrier, which also
-      // orders these tile reads before its writes into the same buffer
-      if constexpr (Sh::S == 1) __syncthreads();
-      C* sm = base + c * SM::stride;
-      fft_line<Sh, false>(v, sm, t, tw, sync);
-      const int lo = __ldg(a.mask_lo + j), hi = __ldg(a.mask_hi + j);
-      const C pyj = __ldg(static_cast<const C*>(a.py) + j);
-#pragma unroll
-      for (int m = 0; m < E; ++m) {
-        if (m % kLoadChunk == 0) load_fence();
-        const int i = t + T * m;
-        if (i < lo || i >= hi) {
-          const C p = cmul(__ldg(px + i), pyj);
-          v[m] = cmul(p, cscale(v[m], is));
-        } else {
-          v[m] = C{Real(0), Real(0)};
-        }
-      }
-      if constexpr (!LAST) fft_line<Sh, true>(v, sm, t, tw, sync);
-      C* col = static_cast<C*>(a.psi) + (int64_t)b * a.batch_stride + j;
-#pragma unroll
-      for (int m = 0; m < E; ++m) col[(int64_t)(t + T * m) * a.ny] = v[m];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && item + 2 * (int)gridDim.x < items) {
-      fence_proxy_async();
-      issue(item + 2 * gridDim.x, w);
-    }
-  }
-}
-
-
 template <int N>
 constexpr int pipe_lines() { return 256 / Shape<N, float>::T; }
-// Threads per CTA of the pipelined column pass; the grid holds as many
-// persistent CTAs as fit on the SMs.
-#ifndef MSF_COL_PIPE_THREADS
-#define MSF_COL_PIPE_THREADS 256
-#endif
-template <typename Real, int N>
-constexpr int pipe_cols() {
-  int c = 16;
-  while (c > 2 && c * Shape<N, Real>::T > MSF_COL_PIPE_THREADS) c >>= 1;
-  return c;
-}
-
 template <int N>
 cudaError_t row_pipe_launch(const PassArgs& a, int* err, cudaStream_t s) {
   constexpr int L = pipe_lines<N>();
@@ -410,53 +284,11 @@ cudaError_t row_staged_launch(const PassArgs& a, int* err, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <typename Real, int N, bool LAST>
-cudaError_t col_pipe_launch(const PassArgs& a, const CUtensorMap& map, int* err,
-                            cudaStream_t s) {
-  constexpr int CC = pipe_cols<Real, N>();
-  constexpr int CB = (int)sizeof(Cx<Real>);
-  using SM = Smem<Shape<N, Real>, CB, CC, true>;
-  constexpr int RAW = (N * CC > CC * SM::stride ? N * CC : CC * SM::stride);
-  constexpr int smem = 2 * ((RAW + 15) / 16 * 16) * CB;
-  // resident CTAs per SM, found once per device after raising the limit
-  static PerDevice configured;
-  static std::atomic<int> per_sm_dev[64];
-  auto k = col_slice_pipe_kernel<Real, N, CC, LAST>;
-  const int dev = current_device();
-  int per_sm = (dev >= 0 && dev < 64) ? per_sm_dev[dev].load() : 0;
-  if (configured.needed(dev) || per_sm < 1) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, CC * Shape<N, Real>::T, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    if (dev >= 0 && dev < 64) per_sm_dev[dev].store(per_sm);
-    configured.mark(dev);
-  }
-  const int items = a.nb * (a.live_groups ? a.n_live_groups : a.ny / CC);
-  if (items <= 0) return cudaSuccess;
-  const int grid = items < per_sm * sm_count() ? items : per_sm * sm_count();
-  k<<<grid, CC * Shape<N, Real>::T, smem, s>>>(a, map, err);
-  return cudaGetLastError();
-}
-
 }  // namespace
 
-bool pipe_supported(int nx, int ny, bool fp64) {
-  // FP64 tiles of 2048-point columns would be 2 columns (32-byte rows) wide
-  auto ok = [fp64](int n) {
-    return n == 256 || n == 512 || n == 1024 || (!fp64 && n == 2048);
-  };
+bool pipe_supported(int nx, int ny) {
+  auto ok = [](int n) { return n == 256 || n == 512 || n == 1024 || n == 2048; };
   return ok(nx) && ok(ny);
-}
-
-int pipe_cols_for(int nx) {
-  switch (nx) {
-    case 256: return pipe_cols<double, 256>();
-    case 512: return pipe_cols<double, 512>();
-    case 1024: return pipe_cols<double, 1024>();
-  }
-  return 0;
 }
 
 cudaError_t launch_row_split_pipe(const PassArgs& a, int* err, cudaStream_t s) {
@@ -501,46 +333,6 @@ cudaError_t launch_row_split_staged(const PassArgs& a, int* err, cudaStream_t s,
     case 2048: return row_staged_launch<2048, 0>(a, err, s);
   }
   return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_col_slice_pipe(const PassArgs& a, bool last, const void* tensor_map,
-                                  int* err, cudaStream_t s) {
-  const CUtensorMap& m = *static_cast<const CUtensorMap*>(tensor_map);
-  switch (a.nx) {
-    case 256: return last ? col_pipe_launch<double, 256, true>(a, m, err, s) : col_pipe_launch<double, 256, false>(a, m, err, s);
-    case 512: return last ? col_pipe_launch<double, 512, true>(a, m, err, s) : col_pipe_launch<double, 512, false>(a, m, err, s);
-    case 1024: return last ? col_pipe_launch<double, 1024, true>(a, m, err, s) : col_pipe_launch<double, 1024, false>(a, m, err, s);
-  }
-  return cudaErrorInvalidValue;
-}
-
-// Tensor map over a batch of FP64 complex planes [nb*nx rows][ny columns],
-// two 8-byte elements a value, box {cols, min(256, nx)} rows; no multicast,
-// no swizzle.
-cudaError_t encode_column_map(void* psi, int nb, int nx, int ny, void* map_out) {
-  // looked up once per process (a thread-safe static: lanes of the request
-  // loop encode maps from their worker thread)
-  static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
-    cudaDriverEntryPointQueryResult q;
-    void* fn = nullptr;
-    cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-    return (e == cudaSuccess && q == cudaDriverEntryPointSuccess)
-               ? reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn)
-               : nullptr;
-  }();
-  if (!encode) return cudaErrorNotSupported;
-  const int cols = pipe_cols_for(nx);
-  if (!cols) return cudaErrorInvalidValue;
-  const int epc = 2;  // 8-byte elements per complex value
-  cuuint64_t dims[2] = {(cuuint64_t)ny * epc, (cuuint64_t)nx * (cuuint64_t)nb};
-  cuuint64_t strides[1] = {(cuuint64_t)ny * 8 * epc};
-  cuuint32_t box[2] = {(cuuint32_t)(cols * epc), (cuuint32_t)(nx < 256 ? nx : 256)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = encode(static_cast<CUtensorMap*>(map_out), CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, psi,
-                      dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 }  // namespace msf

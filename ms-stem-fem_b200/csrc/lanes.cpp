@@ -75,14 +75,15 @@ msf_status Lane::init() {
   // the same bits; the switch lets tests and benchmarks compare them)
   const char* u = std::getenv("MSF_LANE_GROUPS");
   groups_ok_ = !(u && u[0] == '0');
-  MSF_CUDA(encode_pair_map(psi_.p, B_, nx_, ny_, col_map_));
+  MSF_CUDA(encode_col_map(false, psi_.p, B_, nx_, ny_, col_map_));
   row_.psi = col_.psi = psi_.p;
   row_.batch_stride = col_.batch_stride = plane_;
   row_.nb = col_.nb = B_;
   row_.nx = col_.nx = nx_;
   row_.ny = col_.ny = ny_;
-  MSF_TRY(ctx_->twiddles(ny_, false, &row_.tw));
-  MSF_TRY(ctx_->col_twiddles(nx_, &col_.tw));
+  MSF_TRY(ctx_->slice_twiddles(false, nx_, ny_, &row_.tw, &col_.tw));
+  // tables filled on the context's stream are read on the lane's
+  MSF_CUDA(cudaStreamSynchronize(ctx_->stream));
   row_.slots = col_.slots = static_cast<const SlotPass*>(table_.p);
   row_.prefetch_tables = (ctx_->pipe & MSF_ROW_PREFETCH) ? 1 : 0;
   slot_.assign(B_, Slot{});
@@ -124,7 +125,7 @@ msf_status Lane::add(SlotJob* job) {
                                cudaMemcpyDeviceToDevice, stream_));
       h_live_ = spec->h_live_groups;
       h_dead_cols_.assign(ny_, 0);
-      const int T = row_line_threads(ny_, false);
+      const int T = row_line_threads(ny_);
       for (int t = 0; t < T; ++t)
         for (int m = 0; m < ny_ / T; ++m)
           if ((spec->h_dead_bits[t] >> m) & 1u) h_dead_cols_[t + T * m] = 1;
@@ -166,7 +167,7 @@ msf_status Lane::add(SlotJob* job) {
 
 msf_status Lane::launch_passes() {
   MSF_CUDA(launch_row(false, ROW_SLOTS, row_, stream_));
-  MSF_CUDA(launch_col_pair(col_, false, col_map_, err_.as<int>(), stream_));
+  MSF_CUDA(launch_col_slice(false, false, col_, col_map_, err_.as<int>(), stream_));
   return MSF_OK;
 }
 
@@ -208,10 +209,10 @@ msf_status Lane::launch_group(const SlotJob* job, int s, int base, int nb) {
   alignas(64) unsigned char map[128];
   const void* m = col_map_;
   if (base != 0) {
-    MSF_CUDA(encode_pair_map(col.psi, nb, nx_, ny_, map));
+    MSF_CUDA(encode_col_map(false, col.psi, nb, nx_, ny_, map));
     m = map;
   }
-  MSF_CUDA(launch_col_pair(col, last, m, err_.as<int>(), stream_));
+  MSF_CUDA(launch_col_slice(false, last, col, m, err_.as<int>(), stream_));
   return MSF_OK;
 }
 

@@ -129,20 +129,17 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
   cudaStream_t st = ctx->stream;
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
 
-  const bool pipe_col = !fp64 || (pipe_supported(g.nx, g.ny, true) &&
-                                  (ctx->pipe_for(g.nx, g.ny) & MSF_PIPE_COL));
   alignas(64) unsigned char col_map[128];
-  if (pipe_col) MSF_CUDA(encode_col_map(fp64, psi.p, B, g, col_map));
+  MSF_CUDA(encode_col_map(fp64, psi.p, B, g.nx, g.ny, col_map));
   PassArgs row, col;
   // columns the band limit removes entirely are skipped (same grid, hence
   // the same mask, for every snapshot)
-  const bool skip_dead = pipe_col && snaps[0]->n_live_groups > 0;
+  const bool skip_dead = snaps[0]->n_live_groups > 0;
   row.psi = col.psi = psi.p;
   row.batch_stride = col.batch_stride = plane;
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
-  MSF_TRY(ctx->twiddles(g.ny, fp64, &row.tw));
-  MSF_TRY(ctx->col_twiddles(g.nx, &col.tw));
+  MSF_TRY(ctx->slice_twiddles(fp64, g.nx, g.ny, &row.tw, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.first_scale = g.nxny / g.s;
   const SegmentPlan seg_acc = segment_plan(A, partial.as<double>());
@@ -185,10 +182,10 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
           op = sl == 0 ? ROW_SPLIT_FIRST : ROW_SPLIT;
           row.psi0 = P.psi0_tab.as<float>() + 2 * plane * sl;
         }
-        MSF_CUDA(launch_row(fp64, op, row, st));
+        MSF_CUDA(fp64 ? launch_row64(op, row, st) : launch_row(false, op, row, st));
         col.px = pbase + prop_stride * sl;
         col.py = pbase + prop_stride * sl + cbytes * g.nx;
-        MSF_CUDA(launch_col_slice(fp64, pipe_col, sl + 1 == S, col, col_map, d_err.as<int>(), st));
+        MSF_CUDA(launch_col_slice(fp64, sl + 1 == S, col, col_map, d_err.as<int>(), st));
       }
       SplitK sk;
       if (!fp64) {

@@ -1,8 +1,7 @@
 // Launch tiling autotuner.  The reference plans its FFTs with FFTW_MEASURE
 // and keeps the plans as a wisdom file per grid (tem.cpp:583-616, exported
 // at 1748-1765).  Here what is measured per grid is the tiling of the
-// batched slice passes: probes per launch, whether the FP64 column pass runs
-// as the persistent TMA-pipelined kernel, whether the split-wave row pass
+// batched slice passes: probes per launch, whether the split-wave row pass
 // stages its slice tables in shared memory (or prefetches them into L1), and
 // that row pass's FFT radix
 // schedule (32 elements a thread in two or three stages, or 16 in three;
@@ -51,9 +50,8 @@ msf_status tune(msf_context* ctx, const msf_specimen* spec, msf_tuning* out) {
   if (batches.empty()) batches.push_back(1);
   std::vector<int> pipes{ctx->pipe};
   if (!ctx->pipe_env) {
-    const bool col = ctx->fp64 && pipe_supported(g.nx, g.ny, true);
     const bool staged = !ctx->fp64 && staged_row_supported(g.nx, g.ny);
-    // FP64 column pass plain or pipelined; FP32 row pass plain (with or without
+    // the column pass has one form; FP32 row pass plain (with or without
     // its L1 table and L2 wavefield prefetches, lines by row or by probe)
     // or staged, each on either FFT radix schedule
     std::vector<int> rows{0};
@@ -69,10 +67,7 @@ msf_status tune(msf_context* ctx, const msf_specimen* spec, msf_tuning* out) {
               MSF_ROW_STAGED,
               MSF_ROW_STAGED | MSF_ROW_ALT};
     pipes.clear();
-    std::vector<int> cols{ctx->fp64 ? 0 : MSF_PIPE_COL};  // FP32: one column pass
-    if (col) cols = {0, MSF_PIPE_COL};
-    for (int c : cols)
-      for (int r : rows) pipes.push_back(c | r);
+    for (int r : rows) pipes.push_back(MSF_PIPE_COL | r);
   }
   const int saved_pipe = ctx->pipe;
   ctx->tuned.erase({g.nx, g.ny});  // time_passes then runs ctx->pipe
