@@ -777,6 +777,10 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
       MSF_CUDA(launch_col_slice(true, s + 1 == S, v, map, d_err.as<int>(), ctx->stream));
       P->setup_launches += 2;
     }
+    MSF_CUDA(launch_clear_vacuum(P->psi0k.as<double>(), spec->kx.as<double>(),
+                                 spec->ky.as<double>(), g.nx, g.ny, g.lambda * g.lambda,
+                                 optics->alpha_max * optics->alpha_max, ctx->stream));
+    P->setup_launches += 1;
     int err_flag = 0;
     MSF_CUDA(cudaMemcpyAsync(&err_flag, d_err.p, sizeof(int), cudaMemcpyDeviceToHost,
                              ctx->stream));

@@ -645,8 +645,14 @@ __global__ void scale_kernel(double2* a, int64_t n, double s,
 }
 
 // ------------------------------------------------------- detection -------
+// 2^-l, exactly
+__device__ __forceinline__ double exp2_neg(int l) { return __hiloint2double((1023 - l) << 20, 0); }
+
 // Value of one probe's exit wave at k-space pixel `pix`: the buffer value,
-// plus (split-wave runs) the vacuum part shifted to the probe's position.
+// plus (split-wave runs) the vacuum part shifted to the probe's position.  The
+// vacuum part is exactly zero outside the aperture (clear_vacuum_kernel), so
+// only there is a phase computed; sides are powers of two, so the phases'
+// integers are reduced by masks.
 template <typename Real>
 __device__ __forceinline__ double2 exit_value(const Cx<Real>* __restrict__ p, int pix,
                                               const SplitK& sk, int sx, int sy) {
@@ -655,10 +661,11 @@ __device__ __forceinline__ double2 exit_value(const Cx<Real>* __restrict__ p, in
   if (sk.psi0k) {
     const double2 z = __ldg(reinterpret_cast<const double2*>(sk.psi0k) + pix);
     if (z.x != 0.0 || z.y != 0.0) {
-      const int mx = pix / sk.ny, my = pix - mx * sk.ny;
+      const int lx = 31 - __clz(sk.nx), ly = 31 - __clz(sk.ny);
+      const int mx = pix >> ly, my = pix & (sk.ny - 1);
       // e^{-2 pi i (mx sx / nx + my sy / ny)} from exact integer phases
-      const double f = (double)(((int64_t)mx * sx) % sk.nx) / sk.nx +
-                       (double)(((int64_t)my * sy) % sk.ny) / sk.ny;
+      const double f = (double)((mx * sx) & (sk.nx - 1)) * exp2_neg(lx) +
+                       (double)((my * sy) & (sk.ny - 1)) * exp2_neg(ly);
       double sn, cs;
       sincospi(-2.0 * f, &sn, &cs);
       x += z.x * cs - z.y * sn;
@@ -666,6 +673,22 @@ __device__ __forceinline__ double2 exit_value(const Cx<Real>* __restrict__ p, in
     }
   }
   return make_double2(x, y);
+}
+
+// The vacuum exit wave is zero outside the aperture (the probe is, and vacuum
+// propagation is a product in k-space), but the transforms that carried it
+// through the slices leave rounding there, for which every pixel of every probe
+// then computed a phase: detection of 256 probes at 1024^2 took 2.0 ms for the
+// ring sums and 2.2 ms for the pixel sums, 0.81 and 0.94 ms with it cleared.
+__global__ void clear_vacuum_kernel(double2* __restrict__ psi0k, const double* __restrict__ kx,
+                                    const double* __restrict__ ky, int nx, int ny, double lsq,
+                                    double amax_sq) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= ny) return;
+  const double kyj = ky[j];
+  for (int i = blockIdx.y; i < nx; i += gridDim.y)  // the test of probe_synth_kernel
+    if (!(__dmul_rn(lsq, ksq_exact(kx[i], kyj)) < amax_sq))
+      psi0k[(int64_t)i * ny + j] = make_double2(0.0, 0.0);
 }
 
 // Sum of a block's values into lane 0 of warp 0 (fixed order).
@@ -1428,6 +1451,14 @@ cudaError_t launch_strided_accumulate(double* dst, int64_t dst_stride, const dou
   if (n <= 0) return cudaSuccess;
   strided_accumulate_kernel<<<blocks_for(n, 128), 128, 0, s>>>(dst, dst_stride, src, src_stride,
                                                                  n, divisor);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_clear_vacuum(double* psi0k, const double* kx, const double* ky, int nx, int ny,
+                                double lsq, double amax_sq, cudaStream_t s) {
+  const int threads = std::min(ny, 256);
+  clear_vacuum_kernel<<<dim3((ny + threads - 1) / threads, std::min(nx, 1024)), threads, 0, s>>>(
+      reinterpret_cast<double2*>(psi0k), kx, ky, nx, ny, lsq, amax_sq);
   return cudaGetLastError();
 }
 

@@ -341,6 +341,11 @@ cudaError_t launch_mtf_magnitude(bool fp64, const void* psi, int64_t stride, int
 cudaError_t launch_mtf_multiply(double* psi, const double* mtf, int64_t plane, int nb,
                                 double inv_s, cudaStream_t s);
 
+// Zero a vacuum exit wave (k-space) outside the aperture lsq k^2 < amax_sq, the
+// probe's own test.
+cudaError_t launch_clear_vacuum(double* psi0k, const double* kx, const double* ky, int nx, int ny,
+                                double lsq, double amax_sq, cudaStream_t s);
+
 // out[p] = sum over r < world of in[r * n + p], added in rank order (FP64):
 // the pixel sums of a sharded raster, the same bits on every rank.
 cudaError_t launch_rank_sum(const double* in, int world, int64_t n, double* out,

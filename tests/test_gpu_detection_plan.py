@@ -59,3 +59,21 @@ def test_pixel_modes_equal_host_finish(nx, ny, box, precision):
         assert np.array_equal(got.v[m], v, equal_nan=True), m
     assert np.array_equal(got.mean_amplitude, want.mean_amplitude)
     assert np.array_equal(got.mean_intensity, want.mean_intensity)
+
+
+# The vacuum part of an FP32 exit wave: its phases come from masked integers and
+# it is kept inside the aperture only.  Long and short sides both ways, shifts
+# up to nearly a side; apertures of one pixel, of some, and past the band limit.
+# FP32 rounds the scattered part alone: log2(N) eps = 7e-7 a transform, 4
+# transforms a slice, 2 slices, 6e-6 if every error added up.
+@pytest.mark.parametrize("nx,ny", [(64, 64), (64, 4096), (4096, 64), (256, 128)])
+@pytest.mark.parametrize("alpha", [1e-5, 0.010, 1.0])
+def test_fp32_exit_wave_matches_fp64(nx, ny, alpha):
+    waves = []
+    for precision in ("fp32", "fp64"):
+        ctx, spec, optics, raster, det, keep = _setup(nx, ny, (nx * 0.1, ny * 0.1), precision,
+                                                      msf.OUT_ADF_IMAGE, 0.04, 0.2)
+        optics.alpha_max = alpha
+        waves.append(ctx.run(spec, optics, raster, det, want_final_psi=True).final_psi_2d)
+    err = np.linalg.norm(waves[0] - waves[1]) / np.linalg.norm(waves[1])
+    assert err < 1e-5, err
