@@ -77,3 +77,22 @@ def test_fp32_exit_wave_matches_fp64(nx, ny, alpha):
         waves.append(ctx.run(spec, optics, raster, det, want_final_psi=True).final_psi_2d)
     err = np.linalg.norm(waves[0] - waves[1]) / np.linalg.norm(waves[1])
     assert err < 1e-5, err
+
+
+# Ring, annulus and pixel sums gather several pixels or probes at a time: counts
+# that are no multiple of them (1, 3, 5, 6 probes; short rings), each against the
+# same sums of one probe at a time, which add the same values in the same order
+# within a segment (exact) and the probes' planes in raster order (1e-14 of FP64
+# rounding for 6 of them).
+@pytest.mark.parametrize("nx,ny,box", [(64, 64, (6.4, 6.4)), (256, 128, (25.6, 12.8))])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("n", [1, 3, 5, 6])
+def test_sums_of_a_batch_equal_single_probes(nx, ny, box, precision, n):
+    outputs = msf.OUT_ADF_IMAGE | msf.OUT_V_RE | msf.OUT_OMEGA_VIMAGE
+    ctx, spec, optics, raster, det, keep = _setup(nx, ny, box, precision, outputs, 0.04, 0.2)
+    whole = ctx.run_partial(spec, optics, raster, det, 0, n)
+    one = [ctx.run_partial(spec, optics, raster, det, k, k + 1) for k in range(n)]
+    for key in ("amp", "inten"):
+        assert np.array_equal(whole[key], np.concatenate([o[key] for o in one])), key
+    for key in ("acc_a", "acc_i"):
+        np.testing.assert_allclose(whole[key], sum(o[key] for o in one), rtol=1e-14)
