@@ -246,8 +246,9 @@ msf_status msf_probe_noalloc(const msf_grid* grid, const msf_optics* optics,
 typedef struct {
   int32_t nx, ny;             /* grid                                          */
   int32_t batch;              /* probes per launch chosen                      */
-  int32_t pipe;               /* slice-pass variants: bit 0 pipelined column
-                                 pass, bit 1 pipelined row pass, bit 2 row
+  int32_t pipe;               /* slice-pass variants: bit 0 accepted and
+                                 without effect (the column pass has one
+                                 form), bit 1 pipelined row pass, bit 2 row
                                  pass with staged slice tables (FP32), bit 3
                                  the FP32 split-wave row pass on its
                                  alternative FFT radix schedule, bit 4 the
@@ -263,9 +264,8 @@ typedef struct {
 } msf_tuning;
 /* Times the two slice passes of `spec`'s grid (CUDA events, after a
  * warm-up) for each candidate probes-per-launch (8 .. 256, within half the
- * free memory) and each slice-pass variant the grid supports (pipelined
- * column pass or not; for FP32, staged row pass or not, in either FFT radix
- * schedule, and the plain one with or without its L1 and L2 prefetches);
+ * free memory) and each slice-pass variant the grid supports (for
+ * FP32: staged row pass or not, in either FFT radix schedule, and the plain one with or without its L1 and L2 prefetches);
  * records the fastest per probe*slice
  * in the context, where msf_run / msf_run_md / msf_run_partial use it for
  * that grid unless the context's batch or MSF_PIPE fixes the choice. */

@@ -68,8 +68,9 @@ struct DevBuf {
 
 }  // namespace msf
 
-// Slice-pass variants (bit mask): the persistent TMA-pipelined column pass,
-// the persistent pipelined split-wave row pass, and the split-wave row pass
+// Slice-pass variants (bit mask): MSF_PIPE_COL is accepted (stored choices name
+// it) and changes nothing, since the column pass has one form; the persistent
+// pipelined split-wave row pass, and the split-wave row pass
 // with its transmission and vacuum rows staged in shared memory by bulk
 // copies (which takes precedence over MSF_PIPE_ROW).
 constexpr int MSF_PIPE_COL = 1, MSF_PIPE_ROW = 2, MSF_ROW_STAGED = 4;
@@ -95,7 +96,7 @@ struct msf_context {
   bool graphs = true;
   // slice-pass variants (MSF_PIPE_* / MSF_ROW_* bits) for grids the tuner
   // has not measured, overridden by the MSF_PIPE environment variable: the
-  // pipelined column pass and the row pass that prefetches its tables
+  // row pass that prefetches its tables
   // (measured 4 % faster for msf_run at 512^2-2048^2; bit-identical)
   int pipe = MSF_PIPE_COL | MSF_ROW_PREFETCH;
   // slice potentials: 0 FFT convolution for slices of at least 64 atoms,
@@ -177,7 +178,7 @@ struct msf_specimen {
   msf::DevBuf prop;           // [slice] {px[nx], py[ny]} complex, context precision
   msf::DevBuf mask_lo, mask_hi;
   // columns the band limit removes entirely: row-pass zero bits, and the
-  // column groups of the pipelined column pass that keep any column
+  // column groups of the column pass that keep any column
   msf::DevBuf dead_bits, live_groups;
   // the row-pass zero bits in the layout of the alternative FFT schedule of
   // the staged row pass (FP32 contexts; empty when it does not apply)

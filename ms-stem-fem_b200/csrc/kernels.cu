@@ -92,7 +92,7 @@ constexpr int row_lines() {
 
 // Columns per CTA of a column pass: as many as fit MSF_COL_THREADS threads
 // (8 FP64 columns give 128-byte row segments; the FP32 column pass is
-// kernels_col32.cu).
+// kernels_col.cuh).
 template <typename Real, int N>
 constexpr int col_cols() {
   using Sh = Shape<N, Real>;

@@ -121,7 +121,7 @@ struct PassArgs {
   // columns (read them as zero); bit 1, its output there need not be stored
   // (the next pass reads none of it)
   int row_dead_io = 0;
-  // ... so the pipelined column pass skips the column groups that hold only
+  // ... so the column pass skips the column groups that hold only
   // such columns: it walks live_groups[n_live_groups] (nullptr: all groups)
   const int32_t* live_groups = nullptr;
   int n_live_groups = 0;
@@ -203,7 +203,7 @@ bool staged_row_supported(int nx, int ny);
 int staged_row_threads(int ny, int schedule);
 cudaError_t launch_row_split_staged(const PassArgs& a, int* err, cudaStream_t s,
                                     int schedule = 0);
-// ---- the column slice pass (kernels_col.cu), sides 64..4096 ----
+// ---- the column slice pass (kernels_col.cuh), sides 64..4096 ----
 // Up to the next slice, or stopping in k-space when `last`, or per slot when
 // a.slots is set (FP32); a.tw from fill_col_twiddles, `tensor_map` (128 bytes)
 // from encode_col_map over the same batch buffer; *err set to 1 if a copy never

@@ -1,4 +1,4 @@
-"""The column slice pass (kernels_col.cu) and the FP64 row pass
+"""The column slice pass (kernels_col.cuh) and the FP64 row pass
 (kernels_row64.cu) at every length they support: FP32 against the FP64 passes
 of the same raster, FP64 against the plain per-step path.
 
