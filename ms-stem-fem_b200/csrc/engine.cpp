@@ -424,10 +424,10 @@ msf_status build_specimen(msf_context* ctx, const msf_grid* gin, const msf_atoms
     if (spec->n_live_columns < g.ny) {
       const bool fp = ctx->fp64;
       spec->h_dead_bits = bits_of(fp ? row64_threads(g.ny) : row_line_threads(g.ny));
-      spec->h_live_groups = groups_of(col_tile(g.nx, fp));
-      spec->n_live_groups = (int)spec->h_live_groups.size();
+      const std::vector<int32_t> live = groups_of(col_tile(g.nx, fp));
+      spec->n_live_groups = (int)live.size();
       MSF_TRY(upload(ctx, &spec->dead_bits, spec->h_dead_bits));
-      MSF_TRY(upload(ctx, &spec->live_groups, spec->h_live_groups));
+      MSF_TRY(upload(ctx, &spec->live_groups, live));
       if (!fp) {
         const std::vector<int32_t> vac = groups_of(col_tile(g.nx, true));
         spec->n_vac_live_groups = (int)vac.size();

@@ -186,8 +186,7 @@ struct msf_specimen {
   // FP32 contexts: the same for the FP64 passes that build vacuum tables
   msf::DevBuf vac_dead_bits, vac_live_groups;
   int n_vac_live_groups = 0;
-  std::vector<uint32_t> h_dead_bits;  // host copies (slot lanes compare them)
-  std::vector<int32_t> h_live_groups;
+  std::vector<uint32_t> h_dead_bits;  // host copy (slot lanes compare it)
   int n_live_groups = 0, n_live_columns = 0;
   // element ranges of a row that hold live columns (two half-open ranges,
   // even bounds; the whole row when no column is removed or the removed

@@ -123,31 +123,29 @@ msf_status Lane::add(SlotJob* job) {
                                cudaMemcpyDeviceToDevice, stream_));
       MSF_CUDA(cudaMemcpyAsync(live_groups_.p, spec->live_groups.p, spec->live_groups.bytes,
                                cudaMemcpyDeviceToDevice, stream_));
-      h_live_ = spec->h_live_groups;
-      h_dead_cols_.assign(ny_, 0);
-      const int T = row_line_threads(ny_);
-      for (int t = 0; t < T; ++t)
-        for (int m = 0; m < ny_ / T; ++m)
-          if ((spec->h_dead_bits[t] >> m) & 1u) h_dead_cols_[t + T * m] = 1;
+      h_dead_bits_ = spec->h_dead_bits;
       row_.row_dead_bits = dead_bits_.as<uint32_t>();
       col_.live_groups = live_groups_.as<int32_t>();
-      col_.n_live_groups = (int)h_live_.size();
+      col_.n_live_groups = spec->n_live_groups;
       skip_ = true;
     }
-  } else if (skip_ && (spec->n_live_groups == 0 || spec->h_live_groups != h_live_)) {
-    // a raster whose band limit removes other columns: every pass from now
-    // on moves all columns.  The slots in flight hold stale values in the
-    // columns that were skipped, which are zero in the full computation:
-    // write those zeros first.
+  } else if (skip_ && spec->h_dead_bits != h_dead_bits_) {
+    // a raster whose band limit removes other columns (the columns are
+    // compared, not their groups: cells of slightly different aspect keep the
+    // same groups): every pass from now on moves all columns.  The slots in
+    // flight hold stale values in the columns that were skipped, which are
+    // zero in the full computation: write those zeros first.
     MSF_CUDA(cudaStreamSynchronize(stream_));
     if (graph_pass_) {
       cudaGraphExecDestroy(graph_pass_);
       graph_pass_ = nullptr;
     }
+    const int T = row_line_threads(ny_);
+    auto dead = [&](int j) { return (h_dead_bits_[j % T] >> (j / T)) & 1u; };
     for (int j0 = 0; j0 < ny_;) {
-      if (!h_dead_cols_[j0]) { ++j0; continue; }
+      if (!dead(j0)) { ++j0; continue; }
       int j1 = j0;
-      while (j1 < ny_ && h_dead_cols_[j1]) ++j1;
+      while (j1 < ny_ && dead(j1)) ++j1;
       MSF_CUDA(cudaMemset2DAsync(static_cast<char*>(psi_.p) + 8 * (size_t)j0, 8 * (size_t)ny_,
                                  0, 8 * (size_t)(j1 - j0), (size_t)nx_ * B_, stream_));
       j0 = j1;
