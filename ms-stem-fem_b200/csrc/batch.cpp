@@ -42,7 +42,7 @@ int lane_slots(msf_context* ctx, int want, int64_t plane, int lanes, int64_t pro
   // wavefields that fit a block the context's pool already has need no look
   // at the free memory (msf_context::default_batch)
   const int64_t most = std::min(footprint, probes);
-  if (ctx->pool->has((size_t)(8 * plane * most))) return (int)std::max<int64_t>(1, most);
+  if (ctx->pool->has({(size_t)(8 * plane * most)})) return (int)std::max<int64_t>(1, most);
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   const int64_t cap = (int64_t)(0.5 * (double)free_b / std::max(1, lanes)) / (8 * plane);

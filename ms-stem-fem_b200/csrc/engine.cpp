@@ -16,6 +16,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <set>
 
 #include "kernels.h"
 
@@ -71,10 +72,16 @@ void* Pool::take(size_t bytes, size_t* got) {
   return p;
 }
 
-bool Pool::has(size_t bytes) {
+bool Pool::has(const std::vector<size_t>& sizes) {
   std::lock_guard<std::mutex> lock(m);
-  auto it = blocks.lower_bound(bytes);
-  return it != blocks.end() && it->first <= 2 * bytes + (4u << 20);
+  std::multiset<size_t> left;
+  for (const auto& kv : blocks) left.insert(kv.first);
+  for (size_t bytes : sizes) {
+    auto it = left.lower_bound(bytes);
+    if (it == left.end() || *it > 2 * bytes + (4u << 20)) return false;
+    left.erase(it);
+  }
+  return true;
 }
 
 std::recursive_mutex& capture_mutex() {
@@ -174,13 +181,18 @@ msf_status msf_context::twiddles(int n, bool want64, const void** out) {
   return MSF_OK;
 }
 
-int msf_context::default_batch(int64_t block_per_wave, int64_t bytes_per_wave, int64_t probes,
-                               int most) {
-  const int64_t want = std::min<int64_t>(probes, most);
-  if (pool->has((size_t)(block_per_wave * want))) return (int)want;
+int msf_context::default_batch(std::initializer_list<int64_t> buffers, int64_t small,
+                               int64_t probes, int most) {
+  int64_t want = std::min<int64_t>(probes, most), per = 0;
+  for (int64_t b : buffers) per += b;
+  if (budget > 0)
+    want = std::clamp<int64_t>((budget - pool->live) / (per + small), 1, want);
+  std::vector<size_t> sizes;
+  for (int64_t b : buffers) sizes.push_back((size_t)(b * want));
+  if (pool->has(sizes)) return (int)want;
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
-  const int64_t cap = (int64_t)(0.5 * (double)free_b) / bytes_per_wave;
+  const int64_t cap = (int64_t)(0.5 * (double)free_b) / per;
   return (int)std::max<int64_t>(1, std::min<int64_t>(cap, want));
 }
 
@@ -1180,23 +1192,49 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   const size_t cbytes = fp64 ? 16 : 8;
   const int S = P.S, n_seg = P.n_seg;
 
+  // what does not grow with the batch first: the batch takes what is left
+  PassArgs row, col;
+  MSF_TRY(ctx->slice_twiddles(fp64, g.nx, g.ny, &row.tw, &col.tw));
+  DevBuf d_err, first, full;
+  MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
+  if (res->first_psi) MSF_TRY(ctx->alloc(&first, 16 * plane));
+  if (res->final_psi && !fp64 && !P.mtf) MSF_TRY(ctx->alloc(&full, 16 * plane));
   // batch of wavefields: the context's, the tuned one for this grid, or the
-  // default (64 with a detector MTF, whose FP64 planes come on top)
+  // default (64 with a detector MTF, whose FP64 planes come on top), which
+  // gives way to smaller ones where its buffers do not fit
   int B = ctx->batch_for(g.nx, g.ny);
-  if (B <= 0) {
-    const int64_t wave = (int64_t)cbytes * plane;
+  const bool by_default = B <= 0;
+  const int64_t wave = (int64_t)cbytes * plane;
+  const int64_t chunk_sums = sizeof(double) * 2 * std::max(P.n_chunks, 1);
+  if (by_default) {
+    // chunk sums, and a replayed batch's (or the MTF's) segment sums and shifts
+    const int64_t small = chunk_sums + sizeof(double) * (4 * n_seg + 1);
     const int64_t most = P.mtf ? 64 : std::clamp<int64_t>((2LL << 30) / wave, 16, 256);
-    B = ctx->default_batch(wave, wave, n_probes, (int)most);
+    B = P.mtf ? ctx->default_batch({wave, 16 * plane}, small, n_probes, (int)most)
+              : ctx->default_batch({wave}, small, n_probes, (int)most);
   }
   B = (int)std::min<int64_t>(B, n_probes);
-  DevBuf psi, d_partial, mtf_psi, mtf_amp, mtf_int;
-  MSF_TRY(ctx->alloc(&psi, cbytes * plane * B));
-  MSF_TRY(ctx->alloc(&d_partial, sizeof(double) * 2 * B * std::max(P.n_chunks, 1)));
-  if (P.mtf) {
-    MSF_TRY(ctx->alloc(&mtf_psi, 16 * plane * B));
-    MSF_TRY(ctx->alloc(&mtf_amp, sizeof(double) * B * n_seg));
-    MSF_TRY(ctx->alloc(&mtf_int, sizeof(double) * B * n_seg));
-  }
+  DevBuf psi, d_partial, mtf_psi, mtf_amp, mtf_int, stage_shift, stage_amp, stage_int;
+  bool use_graph = false;
+  MSF_TRY(alloc_batch(&B, by_default, [&](int n) -> msf_status {
+    for (DevBuf* b : {&psi, &d_partial, &mtf_psi, &mtf_amp, &mtf_int, &stage_shift, &stage_amp,
+                      &stage_int})
+      b->release();
+    MSF_TRY(ctx->alloc(&psi, wave * n));
+    MSF_TRY(ctx->alloc(&d_partial, chunk_sums * n));
+    if (P.mtf) {
+      MSF_TRY(ctx->alloc(&mtf_psi, 16 * plane * n));
+      MSF_TRY(ctx->alloc(&mtf_amp, sizeof(double) * n * n_seg));
+      MSF_TRY(ctx->alloc(&mtf_int, sizeof(double) * n * n_seg));
+    }
+    use_graph = ctx->graphs && n_probes / n >= 2;
+    if (use_graph) {
+      MSF_TRY(ctx->alloc(&stage_shift, sizeof(int32_t) * 2 * n));
+      MSF_TRY(ctx->alloc(&stage_amp, sizeof(double) * n * n_seg));
+      MSF_TRY(ctx->alloc(&stage_int, sizeof(double) * n * n_seg));
+    }
+    return MSF_OK;
+  }));
   SegmentPlan seg;
   seg.idx = P.seg_idx.as<int32_t>();
   seg.chunk_begin = P.chunk_begin.as<int32_t>();
@@ -1205,19 +1243,16 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   seg.ng = n_seg;
   seg.partial = d_partial.as<double>();
 
-  // persistent TMA-pipelined passes for FP32 grids they support
+  // variants of the FP32 row pass
   const int pipe = ctx->pipe_for(g.nx, g.ny);
   const bool staged_row = !fp64 && staged_row_supported(g.nx, g.ny) && (pipe & MSF_ROW_STAGED);
   const int row_sched = !fp64 && staged_row_supported(g.nx, g.ny) && (pipe & MSF_ROW_ALT) ? 1 : 0;
   const bool pipe_row = !fp64 && !staged_row && !row_sched && pipe_supported(g.nx, g.ny) &&
                         (pipe & MSF_PIPE_ROW);
   alignas(64) unsigned char col_map[128];
-  DevBuf d_err;
-  MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), ctx->stream));
   MSF_CUDA(encode_col_map(fp64, psi.p, B, g.nx, g.ny, col_map));
 
-  PassArgs row, col;
   if (!pipe_row && spec->n_live_groups > 0) {  // skip removed columns
     row.row_dead_bits = spec->dead_bits.as<uint32_t>();
     col.live_groups = spec->live_groups.as<int32_t>();
@@ -1227,7 +1262,6 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
   row.batch_stride = col.batch_stride = plane;
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
-  MSF_TRY(ctx->slice_twiddles(fp64, g.nx, g.ny, &row.tw, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.prefetch_tables = (!fp64 && (pipe & MSF_ROW_PREFETCH)) ? 1 : 0;
   if (!fp64 && !staged_row && row_sched == 0 && !pipe_row && (pipe & MSF_ROW_L2AHEAD))
@@ -1317,15 +1351,7 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
 
   MSF_CUDA(cudaEventRecord(ev0, ctx->stream));
   cudaGraphExec_t graph_exec = nullptr;
-  DevBuf stage_shift, stage_amp, stage_int;
-  const bool use_graph = ctx->graphs && n_probes / B >= 2;
-  if (use_graph) {
-    MSF_TRY(ctx->alloc(&stage_shift, sizeof(int32_t) * 2 * B));
-    MSF_TRY(ctx->alloc(&stage_amp, sizeof(double) * B * n_seg));
-    MSF_TRY(ctx->alloc(&stage_int, sizeof(double) * B * n_seg));
-  }
   msf_status st = MSF_OK;
-  DevBuf first;
   for (int64_t p0 = 0; p0 < n_probes && st == MSF_OK; p0 += B) {
     const int nb = (int)std::min<int64_t>(B, n_probes - p0);
     if (use_graph && nb == B && p0 > 0) {
@@ -1363,7 +1389,6 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
     if (st == MSF_OK && p0 == 0 && res->first_psi) {
       // the first probe's exit wave (adfstem.cpp:2139-2221), before the
       // next batch reuses its buffer
-      MSF_TRY(ctx->alloc(&first, 16 * plane));
       if (fp64)
         MSF_CUDA(cudaMemcpyAsync(first.p, psi.p, 16 * plane, cudaMemcpyDeviceToDevice,
                                  ctx->stream));
@@ -1397,8 +1422,6 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
                                16 * plane, cudaMemcpyDeviceToHost, ctx->stream));
     } else {
       // exit wave = scattered part + the vacuum part at this probe's shift
-      DevBuf full;
-      MSF_TRY(ctx->alloc(&full, 16 * plane));
       const int64_t pl = n_probes - 1;
       MSF_CUDA(launch_assemble_split(psi.as<float>() + 2 * plane * last, P.psi0k.as<double>(),
                                      g.nx, g.ny, P.shifts[2 * pl], P.shifts[2 * pl + 1],

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -37,8 +38,8 @@ struct Pool {
   // A cached block of at least `bytes` and at most twice that (+4 MiB), or
   // nullptr; *got receives its size.
   void* take(size_t bytes, size_t* got);
-  // Whether take() would find one.
-  bool has(size_t bytes);
+  // Whether take() would find a block for each of these, one after the other.
+  bool has(const std::vector<size_t>& sizes);
   // Keeps a released block.  Waits for the device first, as cudaFree does,
   // so that no kernel still in flight on any stream can see it reused.
   void give(void* p, size_t bytes);
@@ -148,11 +149,13 @@ struct msf_context {
   // Wavefields per launch when neither the caller nor the tuner chose: about
   // 2 GiB of them, 16 to 256 (256 at 1024^2 FP32, where a larger launch reads
   // the slice's tables once for more probes: 4 to 5 % faster than 64), at most
-  // `probes` and what half the free memory holds at bytes_per_wave.  A batch
-  // whose largest buffer (block_per_wave a wavefield) fits a block the pool
-  // already has needs no look at the free memory: that call takes 0.1 ms on a
-  // quiet host and has taken 74 ms on a busy one.
-  int default_batch(int64_t block_per_wave, int64_t bytes_per_wave, int64_t probes, int most);
+  // `probes`, what the budget leaves and what half the free memory holds.
+  // buffers: bytes a wavefield of each large buffer of the batch, in the order
+  // of their allocation; small: of the others together.  A batch whose large
+  // buffers all find a block in the pool needs no look at the free memory: that
+  // call takes 0.1 ms on a quiet host and has taken 74 ms on a busy one.
+  int default_batch(std::initializer_list<int64_t> buffers, int64_t small, int64_t probes,
+                    int most);
   // pinned host buffer the per-probe and per-pixel sums of a raster are
   // copied into before the host finish (grown on demand, reused by every
   // raster; freed with the context)
@@ -167,6 +170,20 @@ struct msf_context {
   // the tables of the slice passes of one precision
   msf_status slice_twiddles(bool fp64, int nx, int ny, const void** row, const void** col);
 };
+
+namespace msf {
+// The buffers of a batch of *batch wavefields, by alloc(n), which releases those
+// of an earlier try first.  Where they do not fit and `shrink`, of half as many,
+// and so on: a pool block can count for more than was asked of it, and other
+// contexts share the device.
+template <class F> msf_status alloc_batch(int* batch, bool shrink, F&& alloc) {
+  for (;;) {
+    const msf_status st = alloc(*batch);
+    if (st != MSF_ERR_NOMEM || !shrink || *batch == 1) return st;
+    *batch = (*batch + 1) / 2;
+  }
+}
+}  // namespace msf
 
 struct msf_specimen {
   msf_context* ctx = nullptr;

@@ -108,30 +108,40 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
   const int64_t n_probes = A.n_probes;
   const int n_seg = A.n_seg, n_k = A.n_k;
 
-  // batch: the wavefields, their FP64 average and (MTF) the filtered waves
+  // batch: the wavefields, their FP64 average and (MTF) the filtered waves;
+  // what does not grow with it first
+  PassArgs row, col;
+  MSF_TRY(ctx->slice_twiddles(fp64, g.nx, g.ny, &row.tw, &col.tw));
+  DevBuf d_err;
+  MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
+  int max_chunks = std::max(A.n_chunks, 1);
+  for (const auto& P : plans) max_chunks = std::max(max_chunks, P.n_chunks);
   int B = ctx->batch_for(g.nx, g.ny);
-  if (B <= 0) {
-    const int64_t per = (int64_t)(cbytes + 16 + (A.mtf ? 16 : 0)) * plane;
-    B = ctx->default_batch(16 * plane, per, n_probes, 64);
+  const bool by_default = B <= 0;
+  const int64_t wave = (int64_t)cbytes * plane, average = 16 * plane;
+  if (by_default) {
+    const int64_t small = sizeof(double) * (2 * max_chunks + 3);
+    B = A.mtf ? ctx->default_batch({wave, average, 16 * plane}, small, n_probes, 64)
+              : ctx->default_batch({wave, average}, small, n_probes, 64);
   }
   B = (int)std::min<int64_t>(B, n_probes);
-  int max_chunks = A.n_chunks;
-  for (const auto& P : plans) max_chunks = std::max(max_chunks, P.n_chunks);
-  DevBuf psi, acc, mtf_psi, partial, s_amp, s_int, adf_acc, d_err;
-  MSF_TRY(ctx->alloc(&psi, cbytes * plane * B));
-  MSF_TRY(ctx->alloc(&acc, 16 * plane * B));
-  if (A.mtf) MSF_TRY(ctx->alloc(&mtf_psi, 16 * plane * B));
-  MSF_TRY(ctx->alloc(&partial, sizeof(double) * 2 * B * std::max(max_chunks, 1)));
-  MSF_TRY(ctx->alloc(&s_amp, sizeof(double) * B));
-  MSF_TRY(ctx->alloc(&s_int, sizeof(double) * B));
-  MSF_TRY(ctx->alloc(&adf_acc, sizeof(double) * B));
-  MSF_TRY(ctx->alloc(&d_err, sizeof(int)));
+  DevBuf psi, acc, mtf_psi, partial, s_amp, s_int, adf_acc;
+  MSF_TRY(alloc_batch(&B, by_default, [&](int n) -> msf_status {
+    for (DevBuf* b : {&psi, &acc, &mtf_psi, &partial, &s_amp, &s_int, &adf_acc}) b->release();
+    MSF_TRY(ctx->alloc(&psi, wave * n));
+    MSF_TRY(ctx->alloc(&acc, average * n));
+    if (A.mtf) MSF_TRY(ctx->alloc(&mtf_psi, 16 * plane * n));
+    MSF_TRY(ctx->alloc(&partial, sizeof(double) * 2 * n * max_chunks));
+    MSF_TRY(ctx->alloc(&s_amp, sizeof(double) * n));
+    MSF_TRY(ctx->alloc(&s_int, sizeof(double) * n));
+    MSF_TRY(ctx->alloc(&adf_acc, sizeof(double) * n));
+    return MSF_OK;
+  }));
   cudaStream_t st = ctx->stream;
   MSF_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
 
   alignas(64) unsigned char col_map[128];
   MSF_CUDA(encode_col_map(fp64, psi.p, B, g.nx, g.ny, col_map));
-  PassArgs row, col;
   // columns the band limit removes entirely are skipped (same grid, hence
   // the same mask, for every snapshot)
   const bool skip_dead = snaps[0]->n_live_groups > 0;
@@ -139,7 +149,6 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
   row.batch_stride = col.batch_stride = plane;
   row.nx = col.nx = g.nx;
   row.ny = col.ny = g.ny;
-  MSF_TRY(ctx->slice_twiddles(fp64, g.nx, g.ny, &row.tw, &col.tw));
   row.inv_s = col.inv_s = 1.0 / g.s;
   row.first_scale = g.nxny / g.s;
   const SegmentPlan seg_acc = segment_plan(A, partial.as<double>());
