@@ -155,7 +155,7 @@ msf_status msf_specimen_create(msf_context* ctx, const msf_grid* grid, const msf
 
 msf_status msf_specimen_destroy(msf_specimen* spec) {
   if (spec) {
-    if (spec->ctx) cudaSetDevice(spec->ctx->device);
+    if (spec->device >= 0) cudaSetDevice(spec->device);  // its context may be gone
     delete spec;
   }
   return MSF_OK;

@@ -307,6 +307,7 @@ msf_status build_specimen(msf_context* ctx, const msf_grid* gin, const msf_atoms
   }
   const int64_t n = (int64_t)zz.size();
   spec->ctx = ctx;
+  spec->device = ctx->device;
   spec->g = make_grid(gin->nx, gin->ny, gin->voltage, gin->xperiod * dx, gin->yperiod * dy,
                       gin->zperiod * dz, gin->xmin, gin->ymin, gin->zmin, gin->xperiod,
                       gin->yperiod, gin->zperiod);

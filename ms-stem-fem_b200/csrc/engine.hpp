@@ -187,6 +187,7 @@ template <class F> msf_status alloc_batch(int* batch, bool shrink, F&& alloc) {
 
 struct msf_specimen {
   msf_context* ctx = nullptr;
+  int device = -1;            // the context's (which may be destroyed first)
   msf::Grid g;
   std::vector<double> lower, thickness;
   std::vector<int64_t> counts;
