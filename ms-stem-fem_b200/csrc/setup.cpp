@@ -300,7 +300,7 @@ PixelRuns detector_runs(const Grid& g, double k1, double k2) {
   for (int i = 0; i < g.nx; ++i) {
     auto ksq = [&](int j) { return g.kx[i] * g.kx[i] + g.ky[j] * g.ky[j]; };
     const int a0 = first(0, half, [&](int j) { return ksq(j) > k1; });
-    const int a1 = first(a0, half, [&](int j) { return ksq(j) > k2; });
+    const int a1 = first(a0, half, [&](int j) { return !(ksq(j) <= k2); });
     const int b0 = first(half, g.ny, [&](int j) { return ksq(j) <= k2; });
     const int b1 = first(b0, g.ny, [&](int j) { return !(ksq(j) > k1); });
     for (const auto& e : {std::pair<int, int>{a0, a1}, std::pair<int, int>{b0, b1}})
