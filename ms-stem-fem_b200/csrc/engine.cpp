@@ -1030,6 +1030,7 @@ msf_status finish_raster(msf_context* ctx, const RasterPlan& P, cudaStream_t str
                                P.spec->ky.as<double>(), g.ny, g.lambda * g.lambda,
                                P.optics.alpha_max * P.optics.alpha_max,
                                P.ring_means.as<double>(), stream));
+    if (P.n_k > 0) res->kernel_launches += 1;
     MSF_CUDA(cudaMemcpyAsync(ring_means, P.ring_means.p, sizeof(double) * n_means,
                              cudaMemcpyDeviceToHost, stream));
     ctx->d2h_bytes += (int64_t)(sizeof(double) * n_means);
@@ -1472,8 +1473,7 @@ msf_status raster_sums(msf_context* ctx, const RasterPlan& P, msf_results* res) 
     // the ring sums of the filtered waves)
     res->kernel_launches =
         P.setup_launches +
-        n_batches * (2 * S + 2 + (P.pix_modes ? 1 : 0) + (P.mtf ? 8 + (P.n_k > 0 ? 2 : 0) : 0)) +
-        (P.pix_modes ? 1 : 0);  // the ring means of the finish
+        n_batches * (2 * S + 2 + (P.pix_modes ? 1 : 0) + (P.mtf ? 8 + (P.n_k > 0 ? 2 : 0) : 0));
   }
   return MSF_OK;
 }

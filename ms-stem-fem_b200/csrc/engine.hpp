@@ -269,7 +269,8 @@ msf_status plan_raster(msf_context* ctx, const msf_specimen* spec, const msf_opt
 msf_status download_sums(msf_context* ctx, const RasterPlan& P, cudaStream_t stream,
                          double* amp, double* inten, double* acc_a, double* acc_i);
 // Copies the plan's sums to the host (synchronising `stream`) and finishes
-// the ADF image and FEM statistics in FP64 in the reference's order.
+// the ADF image and FEM statistics in FP64 in the reference's order; adds what it
+// launches to res->kernel_launches.
 msf_status finish_raster(msf_context* ctx, const RasterPlan& plan, cudaStream_t stream,
                          msf_results* res);
 // The ADF image and FEM statistics from per-probe sums of a whole raster

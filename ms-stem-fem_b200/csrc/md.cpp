@@ -252,12 +252,11 @@ msf_status run_md(msf_context* ctx, int n_snap, const msf_specimen* const* snaps
   MSF_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
-  MSF_TRY(finish_raster(ctx, A, st, res));
   res->seconds_raster = 1e-3 * ms;
   res->seconds_setup = 0;
   res->probe_slices = probe_slices;
   res->kernel_launches = launches;
-  return MSF_OK;
+  return finish_raster(ctx, A, st, res);
 }
 
 }  // namespace msf

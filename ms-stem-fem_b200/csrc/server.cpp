@@ -284,7 +284,7 @@ struct msf_server {
     if (s.status == MSF_OK) s.status = r.lane->check_error();
     if (s.status != MSF_OK) s.error = last_error_copy();
     s.probe_slices = P.n_probes * P.S;
-    s.launches = P.setup_launches + r.lane->launches();
+    s.launches = P.setup_launches + r.lane->launches() + res.kernel_launches;
     s.seconds_setup = r.setup_s;
     s.latency = now_s() - r.t_submit;
     s.seconds_raster = now_s() - r.t_admit;
