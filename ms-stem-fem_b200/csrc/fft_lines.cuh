@@ -8,15 +8,36 @@
 //
 // A radix-R stage after NS-point sub-transforms computes
 //   X[k + NS m] = sum_r v[r] W_(NS R)^(r (k + NS m))
-// by log2 R decimation-in-time layers: the layer of block size B pairs m and
-// m + B/2 with the twiddle W_(NS B)^(k + NS m), so the stage's own twiddles
-// cost nothing beyond the butterflies' (a separate multiply before an
-// untwiddled DFT costs one more complex product an element).  A butterfly is
-//   r = a + w b (four FMAs),  q = 2 a - r (two),
-// six instead of the four multiplies and four adds of product, sum and
-// difference.  m >= B/4 needs no twiddle of its own: it is -i times that of
-// m - B/4.  A stage of radix 32 then reads 16 twiddles per thread and two
-// lines where the product form reads 31 per line.
+// in one of two forms:
+//
+//  * product: v[r] W_(NS R)^(r k), R - 1 table entries, then an untwiddled
+//    butterfly (32 points as 4 x 8, 16 as 4 x 4).  Every first stage is this one,
+//    without the product.
+//  * fused: log2 R decimation-in-time layers; the layer of block size B pairs m
+//    and m + B/2 with the twiddle W_(NS B)^(k + NS m), so the stage's own
+//    twiddles cost nothing beyond the butterflies'.  A butterfly is
+//    r = a + w b (four FMAs), q = 2 a - r (two); m >= B/4 needs no twiddle of
+//    its own, it is -i times that of m - B/4.  Half the entries of the other
+//    form, but every layer multiplies, and q inherits the rounding of r.
+//
+// Which form a length takes is a matter of rounding first.  Exit waves' rms error
+// outside the aperture against FP64 (FP32) and long double (FP64); first with the
+// schedules of fft_core.cuh, products throughout, then with every stage fused and
+// q = 2 a - r, then as it is here:
+//   FP32, 1e-7:  64^2 4.33 4.93 4.32   128^2 6.42 7.29 6.41   256^2 6.86 7.41 6.87
+//                512^2 7.57 7.73 7.55  1024^2 9.12 8.75 8.28  2048^2 5.24 5.62 5.24
+//                4096 x 64 7.48 7.45 6.80
+//   FP64, 1e-12: 64^2 0.43 0.47 0.41   128^2 1.69 1.74 1.31   256^2 1.90 2.84 1.85
+//                512^2 8.06 8.17 5.97  1024^2 18.1 17.8 12.7  2048 x 64 6.44 7.02 4.90
+// (part of the FP64 gain is the tables', see line_twiddles).  Stages are fused
+// where that error is no larger and it is the faster form: FP64 rows of 512 points
+// 1.69 us a probe against 3.57, 1024 6.4 against 12.1, 2048 39.8 against 47.4, 4096
+// 181 against 231 (at 32 elements a thread the product form's table reads are
+// exposed); FP32 columns of 4096 points 70.9 against 73.2, 1024 2.77 against 2.78.  At
+// 2048 points fused later stages round 0.5 % worse (5.26), at 512 better (7.27) but
+// take 0.735 us against 0.72.  Elsewhere the product form costs 1 to 4 % of a column
+// pass (FP32 2048^2 13.3 -> 13.7 us a probe, 512^2 0.71 -> 0.72, 128^2 0.074 -> 0.076)
+// and more of the FP64 rows of 128 and 256 points (0.098 -> 0.106, 0.338 -> 0.403 us).
 #pragma once
 #include <cmath>
 #include <vector>
@@ -56,13 +77,13 @@ template <int N_, int E_, int R0_, int R1_, int R2_ = 1> struct LineShape {
   __host__ __device__ static constexpr int ns(int s) {
     return s == 0 ? 1 : s == 1 ? R0_ : R0_ * R1_;
   }
-  // entries of one butterfly's twiddles: one for B = 2 and 4, B/4 after
-  __host__ __device__ static constexpr int tw_rows(int r) {
-    return r <= 2 ? r / 2 : r == 4 ? 2 : tw_rows(r / 2) + r / 4;
+  // entries of one butterfly's twiddles: fused, one for B = 2 and 4 and B/4 after
+  __host__ __device__ static constexpr int tw_rows(int r, bool fused) {
+    return !fused ? r - 1 : r <= 2 ? r / 2 : r == 4 ? 2 : tw_rows(r / 2, true) + r / 4;
   }
   // stage s >= 1's table [row][k], k < ns(s), after the earlier stages'
-  __host__ __device__ static constexpr int tw_off(int s) {
-    return s <= 1 ? 0 : tw_off(s - 1) + tw_rows(radix(s - 1)) * ns(s - 1);
+  __host__ __device__ static constexpr int tw_off(int s, bool fused) {
+    return s <= 1 ? 0 : tw_off(s - 1, fused) + tw_rows(radix(s - 1), fused) * ns(s - 1);
   }
 };
 // columns: the fewest stages
@@ -82,18 +103,32 @@ template <> struct RowShapeOf<2048> { using type = LineShape<2048, 16, 16, 16, 8
 template <> struct RowShapeOf<4096> { using type = LineShape<4096, 16, 16, 16, 16>; };
 template <int N> using RowShape = typename RowShapeOf<N>::type;
 
-// A shape's twiddles w_(NS B)^(k + NS m), stage by stage in the order the
-// layers read them, (cos, -sin) pairs computed in FP64.
+// Whether a length's twiddled stages are fused (see the head of the file).
+template <typename Real, int N> __host__ __device__ constexpr bool fused_twiddles() {
+  return sizeof(Real) == 4 ? N == 1024 || N == 4096 : N >= 512;
+}
+
+// A shape's twiddles, stage by stage in the order they are read, (cos, -sin)
+// pairs.  In long double: an FP64 angle near 2 pi carries a rounding several times
+// the entry's own.
 template <class Sh, typename Real> void line_twiddles(std::vector<Real>& out) {
-  const double two_pi = 6.283185307179586476925286766559;
-  for (int s = 1; s < Sh::S; ++s)
-    for (int B = 2; B <= Sh::radix(s); B *= 2)
-      for (int m = 0; m < (B > 4 ? B / 4 : 1); ++m)
-        for (int k = 0; k < Sh::ns(s); ++k) {
-          const double x = two_pi * (k + (double)Sh::ns(s) * m) / ((double)Sh::ns(s) * B);
-          out.push_back((Real)std::cos(x));
-          out.push_back((Real)-std::sin(x));
-        }
+  const long double two_pi = 6.283185307179586476925286766559005768L;
+  auto put = [&](int num, int den) {
+    const long double x = two_pi * num / den;
+    out.push_back((Real)std::cos(x));
+    out.push_back((Real)-std::sin(x));
+  };
+  for (int s = 1; s < Sh::S; ++s) {
+    const int R = Sh::radix(s), NS = Sh::ns(s);
+    if (fused_twiddles<Real, Sh::N>()) {
+      for (int B = 2; B <= R; B *= 2)
+        for (int m = 0; m < (B > 4 ? B / 4 : 1); ++m)
+          for (int k = 0; k < NS; ++k) put(k + NS * m, NS * B);
+    } else {
+      for (int r = 1; r < R; ++r)
+        for (int k = 0; k < NS; ++k) put(r * k, NS * R);
+    }
+  }
 }
 
 // Table entries from global or shared memory.
@@ -173,27 +208,6 @@ __device__ __forceinline__ void bfly(Pair& a, Pair& b, float c, float s) {
     b = q;
   }
 }
-// w = 1
-__device__ __forceinline__ void bfly_1(Pair& a, Pair& b) {
-  const Pair r{f2add(a.re, b.re), f2add(a.im, b.im)};
-  b = Pair{f2sub(a.re, b.re), f2sub(a.im, b.im)};
-  a = r;
-}
-// w = -i (forward) or +i (inverse)
-template <bool INV>
-__device__ __forceinline__ void bfly_i(Pair& a, Pair& b) {
-  Pair r, q;
-  if constexpr (INV) {
-    r = Pair{f2sub(a.re, b.im), f2add(a.im, b.re)};
-    q = Pair{f2add(a.re, b.im), f2sub(a.im, b.re)};
-  } else {
-    r = Pair{f2add(a.re, b.im), f2sub(a.im, b.re)};
-    q = Pair{f2sub(a.re, b.im), f2add(a.im, b.re)};
-  }
-  a = r;
-  b = q;
-}
-
 template <bool INV, int NEED = 3>
 __device__ __forceinline__ void bfly(double2& a, double2& b, double c, double s0) {
   const double s = INV ? -s0 : s0;
@@ -205,72 +219,144 @@ __device__ __forceinline__ void bfly(double2& a, double2& b, double c, double s0
     b = make_double2(fma(s, b.y, fma(-c, b.x, a.x)), fma(-s, b.x, fma(-c, b.y, a.y)));
   }
 }
-__device__ __forceinline__ void bfly_1(double2& a, double2& b) {
-  const double2 r = cadd(a, b);
-  b = csub(a, b);
-  a = r;
-}
-template <bool INV>
-__device__ __forceinline__ void bfly_i(double2& a, double2& b) {
-  const double2 w = INV ? make_double2(-b.y, b.x) : make_double2(b.y, -b.x);
-  const double2 r = cadd(a, w);
-  b = csub(a, w);
-  a = r;
-}
-
-// Layers B, 2B, .. R of a stage's butterfly over u[0..R) (bit-reversed in,
-// natural out).  k: this butterfly's first entry of the table tw, rows NS apart.
-// ZIN: E slots' dead range is zero on entry (first layer of the first stage,
-// slot of u[bitrev(r)] = r, R = E); ZOUT: not needed on exit (last layer).
-template <int R, int B, int NS, bool INV, bool ZIN, bool ZOUT, int NB, int BI, class V, class Tw>
-__device__ __forceinline__ void line_layers(V (&u)[R], const Tw& tw, int k) {
+// Layers B, 2B, .. R of a fused stage over u[0..R) (bit-reversed in, natural
+// out).  k: this butterfly's first entry of the table tw, rows NS apart.  ZOUT: E
+// slots' dead range is not needed on exit (last layer).
+template <int R, int B, int NS, bool INV, bool ZOUT, int NB, int BI, class V, class Tw>
+__device__ __forceinline__ void fused_layers(V (&u)[R], const Tw& tw, int k) {
   if constexpr (B <= R) {
     constexpr int H = B / 2;
     constexpr int ROWS = H >= 2 ? H / 2 : 1;  // twiddles of this layer
     constexpr int ROW0 = B == 2 ? 0 : B == 4 ? 1 : B / 4;
     typename Tw::type w[ROWS];
-    if constexpr (NS > 1) {
 #pragma unroll
-      for (int m = 0; m < ROWS; ++m) w[m] = tw(k + (ROW0 + m) * NS);
-    }
+    for (int m = 0; m < ROWS; ++m) w[m] = tw(k + (ROW0 + m) * NS);
     sfor<0, R, B>([&](auto baseI) {
       sfor<0, H>([&](auto mI) {
         constexpr int base = decltype(baseI)::value, m = decltype(mI)::value;
         V& a = u[base + m];
         V& b = u[base + m + H];
-        if constexpr (NS == 1) {
-          if constexpr (ZIN && B == 2) {
-            constexpr int ra = bitrev(base, ilog2(R)), rb = bitrev(base + 1, ilog2(R));
-            if constexpr (dead_slot<R>(ra) && dead_slot<R>(rb)) {
-            } else if constexpr (dead_slot<R>(rb)) {
-              b = a;
-            } else if constexpr (dead_slot<R>(ra)) {
-              a = b;
-              b = vneg(b);
-            } else {
-              bfly_1(a, b);
-            }
-          } else if constexpr (m == 0) {
-            bfly_1(a, b);
-          } else if constexpr (4 * m == B) {
-            bfly_i<INV>(a, b);
-          } else {
-            using Real = typename LineOf<V>::Real;
-            constexpr Real c = (Real)cos64(m * (64 / B)), s = (Real)-sin64(m * (64 / B));
-            bfly<INV>(a, b, c, s);
-          }
-        } else {
-          // outputs of the last layer: element slots BI + NB m
-          constexpr int E = R * NB;
-          constexpr int need = !(ZOUT && B == R) ? 3
-                               : (dead_slot<E>(BI + NB * m) ? 0 : 1) |
-                                     (dead_slot<E>(BI + NB * (m + H)) ? 0 : 2);
-          if constexpr (m < ROWS) bfly<INV, need>(a, b, w[m].x, w[m].y);
-          else bfly<INV, need>(a, b, w[m - ROWS].y, -w[m - ROWS].x);  // -i w
-        }
+        // outputs of the last layer: element slots BI + NB m
+        constexpr int E = R * NB;
+        constexpr int need = !(ZOUT && B == R) ? 3
+                             : (dead_slot<E>(BI + NB * m) ? 0 : 1) |
+                                   (dead_slot<E>(BI + NB * (m + H)) ? 0 : 2);
+        if constexpr (m < ROWS) bfly<INV, need>(a, b, w[m].x, w[m].y);
+        else bfly<INV, need>(a, b, w[m - ROWS].y, -w[m - ROWS].x);  // -i w
       });
     });
-    line_layers<R, 2 * B, NS, INV, ZIN, ZOUT, NB, BI>(u, tw, k);
+    fused_layers<R, 2 * B, NS, INV, ZOUT, NB, BI>(u, tw, k);
+  }
+}
+
+__device__ __forceinline__ Pair cadd(const Pair& a, const Pair& b) {
+  return Pair{f2add(a.re, b.re), f2add(a.im, b.im)};
+}
+__device__ __forceinline__ Pair csub(const Pair& a, const Pair& b) {
+  return Pair{f2sub(a.re, b.re), f2sub(a.im, b.im)};
+}
+// a * w (INV: its conjugate), the same w for both lines
+template <bool INV> __device__ __forceinline__ Pair twiddle(const Pair& a, float2 w) {
+  const float2 C = f2(w.x), S = f2(INV ? -w.y : w.y);
+  return Pair{f2fma(C, a.re, f2mul(f2neg(S), a.im)), f2fma(C, a.im, f2mul(S, a.re))};
+}
+template <bool INV> __device__ __forceinline__ double2 twiddle(const double2& a, double2 w) {
+  return INV ? cmulc(a, w) : cmul(a, w);
+}
+template <int K, int M, bool INV> __device__ __forceinline__ Pair twc(const Pair& a) {
+  constexpr int k = (K * (64 / M)) & 63;
+  if constexpr (k == 0) return a;
+  else if constexpr (k == 16) return INV ? Pair{f2neg(a.im), a.re} : Pair{a.im, f2neg(a.re)};
+  else if constexpr (k == 32) return vneg(a);
+  else if constexpr (k == 48) return INV ? Pair{a.im, f2neg(a.re)} : Pair{f2neg(a.im), a.re};
+  else return twiddle<INV>(a, make_float2((float)cos64(k), (float)-sin64(k)));
+}
+// x, y <- x + y, x - y; DX, DY: x, y is zero
+template <bool DX, bool DY, class V> __device__ __forceinline__ void sum_diff(V& x, V& y) {
+  if constexpr (DX && DY) {
+  } else if constexpr (DY) {
+    y = x;
+  } else if constexpr (DX) {
+    x = y;
+    y = vneg(y);
+  } else {
+    const V t = cadd(x, y);
+    y = csub(x, y);
+    x = t;
+  }
+}
+// Radix-2 decimation-in-frequency layers over u[OFF + r STR], r < R (natural order
+// in, bit-reversed out).  Z: the dead slots of u are zero.
+template <int R, int OFF, int STR, bool INV, bool Z, class V, int E>
+__device__ __forceinline__ void line_dif(V (&u)[E]) {
+  if constexpr (R > 1) {
+    constexpr int H = R / 2;
+    sfor<0, H>([&](auto kI) {
+      constexpr int k = decltype(kI)::value, x = OFF + k * STR, y = OFF + (k + H) * STR;
+      sum_diff<Z && dead_slot<E>(x), Z && dead_slot<E>(y)>(u[x], u[y]);
+      u[y] = twc<k, R, INV>(u[y]);
+    });
+    line_dif<H, OFF, STR, INV, false>(u);
+    line_dif<H, OFF + H * STR, STR, INV, false>(u);
+  }
+}
+// DFT of u, natural order in; out(k) names the slot that holds output k.  32
+// points as 4 x 8 and 16 as 4 x 4 (fft_core.cuh).
+template <int R> __host__ __device__ constexpr int dft_out(int k) {
+  if (R < 16) return bitrev(k, ilog2(R));
+  const int R2 = R / 4, k1 = k & 3, k2 = k >> 2;
+  return R2 * bitrev(k1, 2) + bitrev(k2, ilog2(R2));
+}
+template <int R, bool INV, bool Z, class V> __device__ __forceinline__ void line_dft(V (&u)[R]) {
+  if constexpr (R < 16) {
+    line_dif<R, 0, 1, INV, Z>(u);
+  } else {
+    constexpr int R2 = R / 4;
+    sfor<0, R2>([&](auto nI) { line_dif<4, decltype(nI)::value, R2, INV, Z>(u); });
+    sfor<1, 4>([&](auto kI) {
+      constexpr int k1 = decltype(kI)::value;
+      sfor<1, R2>([&](auto nI) {
+        constexpr int n2 = decltype(nI)::value, at = R2 * bitrev(k1, 2) + n2;
+        u[at] = twc<(n2 * k1) % R, R, INV>(u[at]);
+      });
+    });
+    sfor<0, 4>([&](auto kI) { line_dif<R2, R2 * decltype(kI)::value, 1, INV, false>(u); });
+  }
+}
+
+// One radix-R butterfly of a stage after NS-point sub-transforms: slots b + r NB
+// of v, which hold its inputs and receive its outputs in natural order.
+template <class Sh, int S, bool INV, bool ZIN, bool ZOUT, int BI, class V, class Tw>
+__device__ __forceinline__ void stage_butterfly(V (&v)[Sh::E], int t, const Tw& tw) {
+  constexpr int E = Sh::E, R = Sh::radix(S), NB = E / R, NS = Sh::ns(S);
+  constexpr bool FUSED = fused_twiddles<typename LineOf<V>::Real, Sh::N>();
+  const int k = (t + Sh::T * BI) & (NS - 1);
+  V u[R];
+  if constexpr (FUSED && NS > 1) {
+    sfor<0, R>([&](auto rI) {
+      constexpr int r = decltype(rI)::value;
+      u[bitrev(r, ilog2(R))] = v[BI + r * NB];
+    });
+    fused_layers<R, 2, NS, INV, ZOUT && S + 1 == Sh::S, NB, BI>(u, tw, Sh::tw_off(S, true) + k);
+    sfor<0, R>([&](auto rI) {
+      constexpr int r = decltype(rI)::value;
+      v[BI + r * NB] = u[r];
+    });
+  } else {
+    u[0] = v[BI];
+    sfor<1, R>([&](auto rI) {
+      constexpr int r = decltype(rI)::value;
+      if constexpr (NS > 1) {
+        u[r] = twiddle<INV>(v[BI + r * NB], tw(Sh::tw_off(S, false) + (r - 1) * NS + k));
+      } else {
+        u[r] = v[BI + r * NB];
+      }
+    });
+    line_dft<R, INV, ZIN && S == 0 && R == E>(u);
+    sfor<0, R>([&](auto rI) {
+      constexpr int r = decltype(rI)::value;
+      v[BI + r * NB] = u[dft_out<R>(r)];
+    });
   }
 }
 
@@ -314,19 +400,7 @@ __device__ __forceinline__ void fft_lines(V (&v)[Sh::E], int t, const Tw& tw, At
       else sync();
     }
     sfor<0, NB>([&](auto bI) {
-      constexpr int b = decltype(bI)::value;
-      const int k = (t + T * b) & (NS - 1);
-      V u[R];
-      sfor<0, R>([&](auto rI) {
-        constexpr int r = decltype(rI)::value;
-        u[bitrev(r, ilog2(R))] = v[b + r * NB];
-      });
-      line_layers<R, 2, NS, INV, ZIN && s == 0 && R == E, ZOUT && s + 1 == Sh::S, NB, b>(
-          u, tw, Sh::tw_off(s) + k);
-      sfor<0, R>([&](auto rI) {
-        constexpr int r = decltype(rI)::value;
-        v[b + r * NB] = u[r];
-      });
+      stage_butterfly<Sh, s, INV, ZIN, ZOUT, decltype(bI)::value>(v, t, tw);
     });
     if constexpr (s + 1 < Sh::S) {
       sfor<0, NB>([&](auto bI) {
@@ -357,19 +431,7 @@ __device__ __forceinline__ void fft_lines_split(V (&v)[Sh::E], int t, const Tw& 
     constexpr int s = decltype(sI)::value;
     constexpr int R = Sh::radix(s), NB = E / R, NS = Sh::ns(s);
     sfor<0, NB>([&](auto bI) {
-      constexpr int b = decltype(bI)::value;
-      const int k = (t + T * b) & (NS - 1);
-      V u[R];
-      sfor<0, R>([&](auto rI) {
-        constexpr int r = decltype(rI)::value;
-        u[bitrev(r, ilog2(R))] = v[b + r * NB];
-      });
-      line_layers<R, 2, NS, INV, ZIN && s == 0 && R == E, ZOUT && s + 1 == Sh::S, NB, b>(
-          u, tw, Sh::tw_off(s) + k);
-      sfor<0, R>([&](auto rI) {
-        constexpr int r = decltype(rI)::value;
-        v[b + r * NB] = u[r];
-      });
+      stage_butterfly<Sh, s, INV, ZIN, ZOUT, decltype(bI)::value>(v, t, tw);
     });
     if constexpr (s + 1 < Sh::S) {
       constexpr int R2 = Sh::radix(s + 1), NB2 = E / R2;

@@ -15,23 +15,27 @@
 //  * up to 512 points, col_ring_kernel: three tile buffers and two groups of
 //    threads that work on different tiles out of step; a tile is transformed
 //    in place and leaves by TMA, the third buffer is in flight meanwhile.
-//    512^2, 256 probes, FP32: 0.171 ms against 0.217 ms for one 16-column tile
-//    of one column per thread behind CTA barriers (4.2 against 3.3 TB/s).  256
-//    points: 0.045 ms, against 0.049 ms for the long-column kernel, which also
-//    loses at 512 (0.189 ms).
+//    512^2, 256 probes, FP32: 0.18 ms against 0.22 ms for one 16-column tile
+//    of one column per thread behind CTA barriers; 256 points: 0.048 against
+//    0.069 ms.  The long-column kernel loses at both (by 10 %).  FP64 tiles of 128
+//    and 256 points take three groups and five buffers.
 //  * from 1024 points, col_wide_kernel: the tile (128 KB) leaves no room for a
 //    second one, so it is read into registers, refilled by TMA at once, and
 //    the transforms exchange half a tile (real parts, then imaginary parts)
-//    at a time through a 64 KB buffer.  FP32, 1024^2, 256 probes: 0.695 ms
-//    against 0.876 ms for two 8-column buffers (64-byte rows); 2048^2, 64
-//    probes, 8 columns: 0.845 against 1.246 ms with 4; 4096^2, 16 probes, 4
-//    columns: 1.15 ms against 4.3 ms for one column per CTA.  Left: the stores
+//    at a time through a 64 KB buffer.  FP32, 1024^2, 256 probes: 0.71 ms
+//    against 0.90 ms for two 8-column buffers (64-byte rows); 2048^2, 64
+//    probes, 8 columns: 0.87 against 1.25 ms with 4; 4096^2, 16 probes, 4
+//    columns: 1.13 ms against 4.4 ms for one column per CTA.  Left: the stores
 //    of a tile leave in one burst behind its last stage, which the next tile's
 //    first loads wait for.
 //
-// FP64, the same kernels, 64 probes: 1024^2 7.9 -> 5.4 us a probe, 512^2 2.36 ->
-// 1.48 and 256^2 0.61 -> 0.46 against a double-buffered TMA pass of half the tile
-// width, 2048^2 68.7 -> 33 against a plain strided one.
+// A batch that does not fill the SMs once pays for the tile copy's latency: up to
+// 16 probes at 64^2 10.9 us a launch against 8.9 with direct loads, at 1024 x 64
+// 19 against 14.6.
+//
+// FP64, the same kernels, us a probe: 1024^2 8.45 -> 5.47, 512^2 2.18 -> 1.42 (64
+// probes), 256^2 0.45 -> 0.33 (256 probes) against a double-buffered TMA pass of
+// half the tile width, 2048^2 67.9 -> 32.7 (16 probes) against a plain strided one.
 //
 // Every wait is bounded: if a phase does not complete within kSpinLimit polls
 // the waiting group records an error in *err and leaves its loop; copies still
@@ -141,28 +145,41 @@ template <class V> __host__ __device__ constexpr int elem_cols() {
 template <class V> __host__ __device__ constexpr int col_words() { return 2 / elem_cols<V>(); }
 
 // --------------------------------------------------- up to 512 points ------
-constexpr int kRingElems = 8, kRingGroups = 2, kRingBufs = 3;  // 128-byte tile rows
+constexpr int kRingElems = 8;  // 128-byte tile rows
 template <int N> __host__ __device__ constexpr int ring_group() {  // threads of a tile
   return kRingElems * ColShape<N>::T;
 }
-// 32 elements take 255 registers a thread (256 threads an SM), 16 take 128
-// (512 threads)
-template <int N> __host__ __device__ constexpr int ring_ctas() {
-  return (ColShape<N>::E >= 32 ? 256 : 512) / (ring_group<N>() * kRingGroups);
+// 32 elements a thread take 255 registers (256 threads an SM), FP32's 16 take 128
+// (512).  FP64's 16 take 168 (384, in three groups): at 128 registers the 256-point
+// pass spills 568 / 628 bytes (stores / loads) and takes 0.464 us a probe, at 168 it
+// spills 72 / 144 and takes 0.332.  What else spills: FP64 128 points 52 / 84, 512
+// points 52 / 100; FP32 128 and 512 points 28 / 52, the slot form of 256 156 / 112.
+template <class V, int N> __host__ __device__ constexpr bool ring_three() {
+  return elem_cols<V>() == 1 && ColShape<N>::E == 16;
 }
-template <int N> __host__ __device__ constexpr int ring_smem() {
-  return kRingBufs * N * kRingElems * 16 + 1024;  // buffers start on 1024 bytes
+template <class V, int N> __host__ __device__ constexpr int ring_groups() {
+  return ring_three<V, N>() ? 3 : 2;
+}
+template <class V, int N> __host__ __device__ constexpr int ring_bufs() {
+  return ring_three<V, N>() ? 5 : 3;
+}
+template <class V, int N> __host__ __device__ constexpr int ring_ctas() {
+  constexpr int threads = ColShape<N>::E >= 32 ? 256 : ring_three<V, N>() ? 384 : 512;
+  return threads / (ring_group<N>() * ring_groups<V, N>());
+}
+template <class V, int N> __host__ __device__ constexpr int ring_smem() {
+  return ring_bufs<V, N>() * N * kRingElems * 16 + 1024;  // buffers start on 1024 bytes
 }
 
 template <class V, int N, bool LAST, bool SLOTS>
-__global__ void __launch_bounds__(ring_group<N>() * kRingGroups, ring_ctas<N>())
+__global__ void __launch_bounds__(ring_group<N>() * ring_groups<V, N>(), ring_ctas<V, N>())
 col_ring_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap, int* err) {
   using Sh = ColShape<N>;
   using Mem = typename LineOf<V>::Mem;
   using C = typename LineOf<V>::C;
   using Real = typename LineOf<V>::Real;
   constexpr int E = Sh::E, T = Sh::T, PC = kRingElems, EC = elem_cols<V>(), COLS = PC * EC;
-  constexpr int G = kRingGroups, GT = ring_group<N>(), NBUF = kRingBufs;
+  constexpr int G = ring_groups<V, N>(), GT = ring_group<N>(), NBUF = ring_bufs<V, N>();
   constexpr int BOX = N < 256 ? N : 256, BUF = N * PC * 16;
   static_assert(T <= 32, "a line's threads share a warp");
   static_assert(NBUF > G, "a buffer is reloaded by its group's next item");
@@ -274,8 +291,8 @@ constexpr int kWideThreads = 256;  // 8192 elements, 32 a thread
 template <int N> __host__ __device__ constexpr int wide_slots() {
   return N + N / ColShape<N>::radix(0);
 }
-template <int N> __host__ __device__ constexpr int wide_tw() {  // twiddles of the length
-  return ColShape<N>::tw_off(ColShape<N>::S);
+template <class V, int N> __host__ __device__ constexpr int wide_tw() {  // twiddles
+  return ColShape<N>::tw_off(ColShape<N>::S, fused_twiddles<typename LineOf<V>::Real, N>());
 }
 template <class V, int N> __host__ __device__ constexpr int wide_base() {
   return N * wide_elems<N>() * 16 + wide_slots<N>() * wide_elems<N>() * 8;
@@ -283,15 +300,15 @@ template <class V, int N> __host__ __device__ constexpr int wide_base() {
 // which tables fit in shared memory too: the twiddles, then the slice's x
 // propagator
 template <class V, int N> __host__ __device__ constexpr bool wide_tw_fits() {
-  return wide_base<V, N>() + wide_tw<N>() * (int)sizeof(typename LineOf<V>::C) <= 226 * 1024;
+  return wide_base<V, N>() + wide_tw<V, N>() * (int)sizeof(typename LineOf<V>::C) <= 226 * 1024;
 }
 template <class V, int N> __host__ __device__ constexpr bool wide_px_fits() {
   return wide_tw_fits<V, N>() &&
-         wide_base<V, N>() + (wide_tw<N>() + N) * (int)sizeof(typename LineOf<V>::C) <= 226 * 1024;
+         wide_base<V, N>() + (wide_tw<V, N>() + N) * (int)sizeof(typename LineOf<V>::C) <= 226 * 1024;
 }
 template <class V, int N> __host__ __device__ constexpr int wide_smem() {
   return wide_base<V, N>() +
-         ((wide_tw_fits<V, N>() ? wide_tw<N>() : 0) + (wide_px_fits<V, N>() ? N : 0)) *
+         ((wide_tw_fits<V, N>() ? wide_tw<V, N>() : 0) + (wide_px_fits<V, N>() ? N : 0)) *
              (int)sizeof(typename LineOf<V>::C);
 }
 
@@ -310,7 +327,7 @@ col_wide_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap, int*
   Mem* tile = reinterpret_cast<Mem*>(smem_raw);
   Half* xb = reinterpret_cast<Half*>(smem_raw + N * PC * 16);
   C* tw_s = reinterpret_cast<C*>(smem_raw + wide_base<V, N>());
-  C* px_s = tw_s + wide_tw<N>();
+  C* px_s = tw_s + wide_tw<V, N>();
   __shared__ uint64_t bar;
   __shared__ int flag;
   const int c = threadIdx.x % PC, t = threadIdx.x / PC;
@@ -334,7 +351,7 @@ col_wide_kernel(const PassArgs a, const __grid_constant__ CUtensorMap tmap, int*
   // buffers leave too little L1 to keep them (0.748 -> 0.695 ms at 1024^2)
   constexpr bool TW_S = wide_tw_fits<V, N>(), PX_S = !SLOTS && wide_px_fits<V, N>();
   if constexpr (TW_S)
-    for (int k = threadIdx.x; k < wide_tw<N>(); k += kWideThreads)
+    for (int k = threadIdx.x; k < wide_tw<V, N>(); k += kWideThreads)
       tw_s[k] = static_cast<const C*>(a.tw)[k];
   if constexpr (PX_S)
     for (int k = threadIdx.x; k < N; k += kWideThreads) px_s[k] = static_cast<const C*>(a.px)[k];
@@ -401,10 +418,10 @@ cudaError_t col_launch(const PassArgs& a, const CUtensorMap& map, int* err, cuda
     k<<<items < sm_count() ? items : sm_count(), kWideThreads, smem, s>>>(a, map, err);
   } else {
     auto k = col_ring_kernel<V, N, LAST, SLOTS>;
-    cudaError_t e = smem_limit_once((const void*)k, ring_smem<N>(), configured);
+    cudaError_t e = smem_limit_once((const void*)k, ring_smem<V, N>(), configured);
     if (e != cudaSuccess) return e;
-    const int resident = ring_ctas<N>() * sm_count();
-    k<<<items < resident ? items : resident, ring_group<N>() * kRingGroups, ring_smem<N>(), s>>>(
+    const int resident = ring_ctas<V, N>() * sm_count();
+    k<<<items < resident ? items : resident, ring_group<N>() * ring_groups<V, N>(), ring_smem<V, N>(), s>>>(
         a, map, err);
   }
   return cudaGetLastError();

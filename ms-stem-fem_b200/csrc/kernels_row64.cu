@@ -9,10 +9,12 @@
 // a thread (255 registers, two radix-32 stages and one exchange) still hide it
 // better than twelve warps of 16 (three stages): 9.3 against 11.8 us a probe, and
 // the transmission row prefetched into L1 during the inverse transform takes
-// that to 6.6.  One 16-element line of three stages with a separate twiddle
-// product took 12.2.  512 points: 2.57 -> 1.69 us, 256: 0.49 -> 0.39 (64 probes).
-// From 2048 points 32 elements spill (59 us a probe) and 16 are the better (58.5
-// -> 38.3 us; 4096: 176 us).
+// that to 6.4.  One 16-element line of three stages with a separate twiddle
+// product took 12.2.  512 points: 2.57 -> 1.69 us (64 probes), 256: 0.44 -> 0.40,
+// 128: 0.122 -> 0.106 (256 probes; the product form of the twiddles, which rounds
+// as little as before, fft_lines.cuh: fused they took 0.34 and 0.098).
+// From 2048 points 32 elements spill (59 us a probe) and 16 are the better (63.7
+// -> 39.8 us; 4096: 362 -> 181).
 #include <algorithm>
 
 #include "fft_lines.cuh"
