@@ -264,10 +264,10 @@ typedef struct {
 } msf_tuning;
 /* Times the two slice passes of `spec`'s grid (CUDA events, after a
  * warm-up) for each candidate probes-per-launch (8 .. 256, within half the
- * free memory) and each slice-pass variant the grid supports (for
- * FP32: staged row pass or not, in either FFT radix schedule, and the plain one with or without its L1 and L2 prefetches);
- * records the fastest per probe*slice
- * in the context, where msf_run / msf_run_md / msf_run_partial use it for
+ * free memory) and each slice-pass variant the grid supports (for FP32:
+ * staged row pass or not, in either FFT radix schedule, and the plain one with
+ * or without its L1 and L2 prefetches); records the fastest per probe*slice in
+ * the context, where msf_run / msf_run_md / msf_run_partial use it for
  * that grid unless the context's batch or MSF_PIPE fixes the choice. */
 msf_status msf_tune(msf_context* ctx, const msf_specimen* spec, msf_tuning* out);
 /* The context's tuning as text, one line per grid ("msf-wisdom 1 <device
