@@ -68,7 +68,7 @@ typedef struct msf_specimen msf_specimen;
 typedef struct {
   int32_t device;          /* CUDA device ordinal                              */
   int32_t precision;       /* msf_precision of wavefields and FFTs             */
-  int32_t batch;           /* probes per launch; 0 = choose from free memory   */
+  int32_t batch;           /* probes per launch; 0 = what fits memory and budget */
   int32_t use_graphs;      /* capture each batch's slice stack in a CUDA graph */
   int64_t hbm_budget;      /* bytes this context may allocate; 0 = no limit    */
 } msf_options;
