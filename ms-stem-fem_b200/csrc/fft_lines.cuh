@@ -29,7 +29,7 @@
 //                4096 x 64 7.48 7.45 6.80
 //   FP64, 1e-12: 64^2 0.43 0.47 0.41   128^2 1.69 1.74 1.31   256^2 1.90 2.84 1.85
 //                512^2 8.06 8.17 5.97  1024^2 18.1 17.8 12.7  2048 x 64 6.44 7.02 4.90
-// (part of the FP64 gain is the tables', see line_twiddles).  Stages are fused
+// (part of the FP64 gain is the tables', see exact_root).  Stages are fused
 // where that error is no larger and it is the faster form: FP64 rows of 512 points
 // 1.69 us a probe against 3.57, 1024 6.4 against 12.1, 2048 39.8 against 47.4, 4096
 // 181 against 231 (at 32 elements a thread the product form's table reads are
@@ -40,6 +40,7 @@
 // and more of the FP64 rows of 128 and 256 points (0.098 -> 0.106, 0.338 -> 0.403 us).
 #pragma once
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "fft_core.cuh"
@@ -108,15 +109,33 @@ template <typename Real, int N> __host__ __device__ constexpr bool fused_twiddle
   return sizeof(Real) == 4 ? N == 1024 || N == 4096 : N >= 512;
 }
 
-// A shape's twiddles, stage by stage in the order they are read, (cos, -sin)
-// pairs.  In long double: an FP64 angle near 2 pi carries a rounding several times
-// the entry's own.
+// (cos, sin) of 2 pi num / den, den a power of two up to 4096, rounded from long
+// double: an FP64 angle near 2 pi carries a rounding several times the entry's own.
+// One octant is evaluated, once in a process (513 pairs of 0.44 us); the rest is
+// its mirror images.
+inline std::pair<double, double> exact_root(int num, int den) {
+  constexpr int N = 4096, O = N / 8;
+  static const std::vector<std::pair<double, double>> octant = [] {
+    std::vector<std::pair<double, double>> t;
+    for (int k = 0; k <= O; ++k) {
+      const long double x = 6.283185307179586476925286766559005768L * k / N;
+      t.emplace_back((double)std::cos(x), (double)std::sin(x));
+    }
+    return t;
+  }();
+  const int k = num * (N / den) % N, o = k / O;
+  const auto& e = octant[o % 2 ? O - k % O : k % O];
+  const bool swap = (o + 1) / 2 % 2;  // octants 1, 2, 5, 6
+  const double c = swap ? e.second : e.first, s = swap ? e.first : e.second;
+  return {o >= 2 && o < 6 ? -c : c, o >= 4 ? -s : s};
+}
+
+// A shape's twiddles, stage by stage in the order they are read, (cos, -sin) pairs.
 template <class Sh, typename Real> void line_twiddles(std::vector<Real>& out) {
-  const long double two_pi = 6.283185307179586476925286766559005768L;
   auto put = [&](int num, int den) {
-    const long double x = two_pi * num / den;
-    out.push_back((Real)std::cos(x));
-    out.push_back((Real)-std::sin(x));
+    const auto [c, s] = exact_root(num, den);
+    out.push_back((Real)c);
+    out.push_back((Real)-s);
   };
   for (int s = 1; s < Sh::S; ++s) {
     const int R = Sh::radix(s), NS = Sh::ns(s);
